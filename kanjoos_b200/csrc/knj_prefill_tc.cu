@@ -179,6 +179,14 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t adesc, uint
           "r"(zero), "r"(zero), "r"(zero), "r"(zero)
         : "memory");
 }
+// one lane of a converged warp (the same one every time)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+// warp of the CTA, known to the compiler to be the same in all its lanes
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 // 16 consecutive f32 columns of this thread's TMEM lane
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   uint32_t r[16];
@@ -261,7 +269,8 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
   constexpr int kStages = S::kStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = warp_index();  // the same register in all lanes: the roles below branch uniformly
   const uint32_t rank = CG == 2 ? cluster_rank() : 0u;  // == blockIdx.x & 1 (m_tiles is even when CG == 2)
 
   // ---- which (expert, token bucket) is this CTA's? scan the counts (E <= 256)
@@ -574,40 +583,44 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
       cp_async_arrive(rank == 0 ? &full[stage] : &locB[stage]);
       KNJ_TC_STAMP(ltr, 64 + 4 * ks + 3);
     }
-  } else if (CG == 2 && warp == 8 && lane == 0 && rank == 1) {
+  } else if (CG == 2 && rank == 1) {
     // =========================== relay (odd CTA) ===========================
     // cp.async completions can only arrive on a barrier of their own CTA: pass them on to the MMA thread
+    if (elect_one())
     for (int ks = 0; ks < nslab && ok; ++ks) {
       const int sb = ks % kStages;
       if (!mbar_spin(&locB[sb], (ks / kStages) & 1, s_fail)) { ok = false; break; }
       mbar_arrive_cluster(cluster_addr(&full[sb], 0));
     }
-  } else if (warp == 8 && lane == 0 && rank == 0) {
+  } else if (elect_one()) {
     // =========================== MMA issue ===========================
-    // Every instruction this thread issues (MMA, commit, barrier test) costs it on the order of a hundred
-    // cycles, and the tensor pipe queues little: what is not an MMA here is idle pipe time. Hence one "full"
-    // barrier per stage for both operands and one commit per CTA.
+    // One elected thread of warp 8. The branch has to be uniform up to elect.sync: picked by `lane == 0` instead, the
+    // same loop took 93 cycles an instruction whatever N was (its operands then have to be moved to uniform registers
+    // one instruction at a time), against N / 2 cycles, the tensor pipe's own rate, this way. Consecutive instructions
+    // alternate between the two accumulators. One "full" barrier per stage covers both operands, one commit the CTA pair.
     const uint32_t idesc = instr_desc_f16(kRowsM * CG, n_mma);
-    for (int ks = 0; ks < nslab && ok; ++ks) {
-      const int st = ks % kStages;
-      if (!mbar_spin(&full[st], (ks / kStages) & 1, s_fail)) { ok = false; break; }
+    const uint64_t a_desc0 = smem_desc_sw128(smem_u32(smem + S::kOffA)), b_desc0 = smem_desc_sw128(smem_u32(smem + S::kOffB));
+    int st = 0;
+    uint32_t par = 0;
+    for (int ks = 0; ks < nslab; ++ks) {
+      if (!mbar_spin(&full[st], par, s_fail)) { ok = false; break; }
       // No proxy fence here: the unpackers fence their own stores before arriving, the gathered rows are
       // complete when their copies' arrivals are (the hand-off CUTLASS' cp.async tcgen05 main loop relies on),
       // and a fence.proxy.async in this thread would wait for the shared-memory reads of every MMA in flight.
       tc_fence_after();
       KNJ_TC_STAMP(blockIdx.x == 0 && ks < 12, 4 * ks + 3);
-      const uint32_t b_addr = smem_u32(smem + S::kOffB + st * S::kBTile);
-      const uint32_t a_addr = smem_u32(smem + S::kOffA + st * NMAT * S::kATile);
+      const uint64_t a_desc = a_desc0 + (uint32_t)(st * NMAT * S::kATile) / 16, b_desc = b_desc0 + (uint32_t)(st * S::kBTile) / 16;
 #pragma unroll
       for (int k = 0; k < kSlabK / 16; ++k) {
 #pragma unroll
-        for (int mat = 0; mat < NMAT; ++mat)  // consecutive instructions alternate between the two accumulators
-          tc_mma_f16<CG>(tmem_base + mat * kMaxTok, smem_desc_sw128(a_addr + mat * S::kATile + k * 32),
-                         smem_desc_sw128(b_addr + k * 32), idesc, (ks > 0 || k > 0) ? 1u : 0u);
+        for (int mat = 0; mat < NMAT; ++mat)
+          tc_mma_f16<CG>(tmem_base + mat * kMaxTok, a_desc + (uint32_t)(mat * S::kATile + k * 32) / 16, b_desc + (uint32_t)(k * 32) / 16, idesc,
+                         (ks > 0 || k > 0) ? 1u : 0u);
       }
       if (CG == 2) tc_commit_pair(smem_u32(&empty[st]));
       else tc_commit_addr<CG>(smem_u32(&empty[st]));
       KNJ_TC_STAMP(blockIdx.x == 0 && ks < 12, 128 + ks);
+      if (++st == kStages) { st = 0; par ^= 1u; }
     }
     if (ok) {
       if (CG == 2) tc_commit_pair(smem_u32(acc_full));
@@ -685,7 +698,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
       if (mat + 1 < kEpiMats) asm volatile("bar.sync 5, 384;" ::: "memory");
     }
   }
-  if (!ok && lane == 0 && p.status) atomicExch(p.status, 1);
+  if (!ok && p.status) atomicExch(p.status, 1);
   tc_fence_before();
   __syncthreads();
   // a CTA of a pair may neither free tensor memory nor leave while the peer still reads its accumulators'
