@@ -132,63 +132,77 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// CTA = 4 warps = 64 tokens x 64 experts; K in steps of 32 through a 3-stage
-// cp.async pipeline (activation tile + router tile per stage).
-template <int DT>
+// CTA = 4 warps; K in steps of 32 through a cp.async pipeline of NSTAGE stages (activation tile + router tile per stage).
+// Every logit is one chain of f32 additions in ascending K whatever the tile, so that near-ties of the routing fall the
+// same way at every token count (K split over warps was faster still, 9 us at 100 and 512 tokens, but changed the sums'
+// order: one near-tie in 16384 tokens fell the other way).
+// MT = 64: 64 tokens x 64 experts, a warp 16 tokens x 64 experts. MT = 16: 16 tokens x 32 experts, a warp 16 tokens x 8.
+// Both are bound by a step's latency over the steps in flight: 64-token tiles with three stages took 36 us for 100 f32
+// rows, 28 us for 512 bf16 rows and 28 us for 4001; the small tiles take 19.5 and 11.5 us, eight stages 22.7 us.
+template <int DT, int MT, int NSTAGE>
+struct RouterTile {
+  static constexpr int kEs = DT == KNJ_DT_F32 ? 4 : 2;  // bytes per activation
+  static constexpr int kExperts = MT == 64 ? 64 : 32;   // per CTA
+  static constexpr int kXTile = MT * 32 * kEs, kWTile = kExperts * 64;  // bytes per stage
+  static constexpr int kBytes = NSTAGE * (kXTile + kWTile);
+};
+template <int DT, int MT, int NSTAGE>
 __global__ void __launch_bounds__(128) router_logits_mma_kernel(const void *__restrict__ x, int64_t ldx,
                                                                 const __nv_bfloat16 *__restrict__ Wr,
                                                                 const float *__restrict__ bias, int T, int H, int E,
                                                                 float *__restrict__ logits) {
-  constexpr int ES = DT == KNJ_DT_F32 ? 4 : 2;      // bytes per activation
+  using S = RouterTile<DT, MT, NSTAGE>;
+  constexpr int ES = S::kEs;
   constexpr int XROW = 32 * ES;                     // bytes per staged activation row
-  constexpr int XTILE = 64 * XROW, WTILE = 64 * 64; // bytes per stage
-  constexpr int STAGES = 3;
-  __shared__ __align__(16) uint8_t sx[STAGES][XTILE];
-  __shared__ __align__(16) uint8_t sw[STAGES][WTILE];
+  constexpr int XTILE = S::kXTile, WTILE = S::kWTile, STAGES = NSTAGE;
+  constexpr int NT = MT == 64 ? 8 : 1;              // 8-expert tiles per warp
+  extern __shared__ __align__(16) uint8_t router_smem[];
+  uint8_t *sx = router_smem, *sw = router_smem + STAGES * XTILE;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int tok0 = blockIdx.y * 64, e0 = blockIdx.x * 64;
+  const int tok0 = blockIdx.y * MT, e0 = blockIdx.x * S::kExperts;
+  const int wrow = MT == 64 ? warp * 16 : 0, wexp = MT == 64 ? 0 : warp * 8;  // this warp's part of the tile
   const int nk = H / 32;
 
   auto issue = [&](int kstep, int st) {
     const int k0 = kstep * 32;
-    // activations: 64 rows x XROW bytes
+    // activations: MT rows x XROW bytes
 #pragma unroll
     for (int c = tid; c < XTILE / 16; c += 128) {
       const int r = c / (XROW / 16), cc = c % (XROW / 16);
       const int tok = tok0 + r;
       const uint8_t *src = static_cast<const uint8_t *>(x) + ((int64_t)min(tok, T - 1) * ldx + k0) * ES + cc * 16;
-      cp_async16(&sx[st][r * XROW + cc * 16], src, tok < T);
+      cp_async16(sx + st * XTILE + r * XROW + cc * 16, src, tok < T);
     }
-    // router rows: 64 experts x 64 bytes
+    // router rows: 64 bytes each
 #pragma unroll
     for (int c = tid; c < WTILE / 16; c += 128) {
       const int r = c >> 2, cc = c & 3;
       const int e = e0 + r;
-      cp_async16(&sw[st][r * 64 + cc * 16], Wr + (size_t)min(e, E - 1) * H + k0 + cc * 8, e < E);
+      cp_async16(sw + st * WTILE + r * 64 + cc * 16, Wr + (size_t)min(e, E - 1) * H + k0 + cc * 8, e < E);
     }
   };
 
-  float acc[8][4];
+  float acc[NT][4];
 #pragma unroll
-  for (int n = 0; n < 8; ++n)
+  for (int n = 0; n < NT; ++n)
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
 
-  issue(0, 0);
-  cp_async_commit();
-  if (nk > 1) issue(1, 1);
-  cp_async_commit();
+  for (int ks = 0; ks < STAGES - 1; ++ks) {
+    if (ks < nk) issue(ks, ks);
+    cp_async_commit();
+  }
   for (int ks = 0; ks < nk; ++ks) {
-    cp_async_wait<1>();
+    cp_async_wait<STAGES - 2>();
     __syncthreads();
-    if (ks + 2 < nk) issue(ks + 2, (ks + 2) % STAGES);
+    if (ks + STAGES - 1 < nk) issue(ks + STAGES - 1, (ks + STAGES - 1) % STAGES);
     cp_async_commit();
     const int st = ks % STAGES;
     // A fragments of rows g and g+8 of this warp's 16 tokens: k = 8t..8t+7 of the 32-wide span
     uint32_t a0[4], a1[4], a2[4], b0[4], b1[4], b2[4];
     auto planes = [&](int row, uint32_t (&p0)[4], uint32_t (&p1)[4], uint32_t (&p2)[4]) {
-      const uint8_t *src = &sx[st][(warp * 16 + row) * XROW + 8 * t * ES];
+      const uint8_t *src = sx + st * XTILE + (wrow + row) * XROW + 8 * t * ES;
       if (DT == KNJ_DT_BF16) {
         const uint4 r = *reinterpret_cast<const uint4 *>(src);
         p0[0] = r.x; p0[1] = r.y; p0[2] = r.z; p0[3] = r.w;
@@ -224,8 +238,8 @@ __global__ void __launch_bounds__(128) router_logits_mma_kernel(const void *__re
     planes(g, a0, a1, a2);
     planes(g + 8, b0, b1, b2);
 #pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      const uint4 w = *reinterpret_cast<const uint4 *>(&sw[st][(n * 8 + g) * 64 + 16 * t]);
+    for (int n = 0; n < NT; ++n) {
+      const uint4 w = *reinterpret_cast<const uint4 *>(sw + st * WTILE + (wexp + n * 8 + g) * 64 + 16 * t);
       mma_bf16_16816(acc[n], a0[0], b0[0], a0[1], b0[1], w.x, w.y);
       mma_bf16_16816(acc[n], a0[2], b0[2], a0[3], b0[3], w.z, w.w);
       if (DT != KNJ_DT_BF16) {
@@ -237,10 +251,10 @@ __global__ void __launch_bounds__(128) router_logits_mma_kernel(const void *__re
     }
   }
   cp_async_wait<0>();
-  const int ra = tok0 + warp * 16 + g, rb = ra + 8;
+  const int ra = tok0 + wrow + g, rb = ra + 8;
 #pragma unroll
-  for (int n = 0; n < 8; ++n) {
-    const int e = e0 + n * 8 + 2 * t;
+  for (int n = 0; n < NT; ++n) {
+    const int e = e0 + wexp + n * 8 + 2 * t;
     const float bb0 = (bias && e < E) ? bias[e] : 0.f, bb1 = (bias && e + 1 < E) ? bias[e + 1] : 0.f;
     if (ra < T && e < E) logits[(size_t)ra * E + e] = acc[n][0] + bb0;
     if (ra < T && e + 1 < E) logits[(size_t)ra * E + e + 1] = acc[n][1] + bb1;
@@ -792,6 +806,36 @@ __global__ void silu_mul_kernel(const float *__restrict__ G, const float *__rest
   }
 }
 
+template <int DT, int MT, int NSTAGE>
+int launch_router_tile(const void *x, int64_t ldx, const __nv_bfloat16 *wr, const float *bias, int T, int H, int E, float *logits,
+                       cudaStream_t st) {
+  using S = RouterTile<DT, MT, NSTAGE>;
+  if (S::kBytes > 48 * 1024) {  // more than the default limit: opt in once per device
+    int dev = 0;
+    KNJ_CUDA(cudaGetDevice(&dev));
+    static bool opted[64] = {false};
+    if (dev < 0 || dev >= 64 || !opted[dev]) {
+      KNJ_CUDA(cudaFuncSetAttribute(router_logits_mma_kernel<DT, MT, NSTAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes));
+      if (dev >= 0 && dev < 64) opted[dev] = true;
+    }
+  }
+  const dim3 grid((E + S::kExperts - 1) / S::kExperts, (T + MT - 1) / MT);
+  router_logits_mma_kernel<DT, MT, NSTAGE><<<grid, 128, S::kBytes, st>>>(x, ldx, wr, bias, T, H, E, logits);
+  return launch_status("router_logits_mma_kernel");
+}
+// Small tiles while they are at most two CTAs an SM (1184 tokens with 128 experts on 148 SMs); then 64-token tiles, eight
+// stages deep while one CTA an SM has to hide its own latency, three where several CTAs of an SM hide one another's (at
+// 16384 tokens eight stages took 55 us, three 47).
+template <int DT>
+int launch_router_logits(const void *x, int64_t ldx, const __nv_bfloat16 *wr, const float *bias, int T, int H, int E,
+                         float *logits, cudaStream_t st) {
+  if ((long long)((T + 15) / 16) * ((E + 31) / 32) <= 2 * sm_count())
+    return launch_router_tile<DT, 16, 8>(x, ldx, wr, bias, T, H, E, logits, st);
+  if ((long long)((T + 63) / 64) * ((E + 63) / 64) <= sm_count())
+    return launch_router_tile<DT, 64, 8>(x, ldx, wr, bias, T, H, E, logits, st);
+  return launch_router_tile<DT, 64, 3>(x, ldx, wr, bias, T, H, E, logits, st);
+}
+
 }  // namespace
 
 extern "C" {
@@ -816,12 +860,10 @@ int knj_router_topk_launch(const void *x, int x_dtype, int64_t ldx, const uint16
   if (T <= 0) return KNJ_OK;
   int rc;
   if (T >= 32 && H % 32 == 0 && ldx % 8 == 0 && aligned16(x)) {
-    dim3 grid((E + 63) / 64, (T + 63) / 64);
     const __nv_bfloat16 *wr = reinterpret_cast<const __nv_bfloat16 *>(Wr_bf16);
-    if (x_dtype == KNJ_DT_BF16) router_logits_mma_kernel<KNJ_DT_BF16><<<grid, 128, 0, as_stream(s)>>>(x, ldx, wr, bias, T, H, E, logits);
-    else if (x_dtype == KNJ_DT_F32) router_logits_mma_kernel<KNJ_DT_F32><<<grid, 128, 0, as_stream(s)>>>(x, ldx, wr, bias, T, H, E, logits);
-    else router_logits_mma_kernel<KNJ_DT_F16><<<grid, 128, 0, as_stream(s)>>>(x, ldx, wr, bias, T, H, E, logits);
-    rc = launch_status("router_logits_mma_kernel");
+    if (x_dtype == KNJ_DT_BF16) rc = launch_router_logits<KNJ_DT_BF16>(x, ldx, wr, bias, T, H, E, logits, as_stream(s));
+    else if (x_dtype == KNJ_DT_F32) rc = launch_router_logits<KNJ_DT_F32>(x, ldx, wr, bias, T, H, E, logits, as_stream(s));
+    else rc = launch_router_logits<KNJ_DT_F16>(x, ldx, wr, bias, T, H, E, logits, as_stream(s));
   } else {
     dim3 grid((E + 7) / 8, (T + kRouterTT - 1) / kRouterTT);
     router_logits_kernel<<<grid, 256, 0, as_stream(s)>>>(x, x_dtype, ldx, reinterpret_cast<const __nv_bfloat16 *>(Wr_bf16),

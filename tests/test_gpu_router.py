@@ -81,3 +81,22 @@ def test_permute_tables(T, E, k):
     act = np.nonzero(hist)[0]
     assert n_active[0] == len(act) and np.array_equal(exp_list[:len(act)], act)
     assert n_active[1] == hist.max()
+
+
+@pytest.mark.parametrize("T,E,dtype", [(32, 128, "f32"), (1183, 128, "bf16"), (1185, 128, "bf16"), (1185, 128, "f32"),
+                                       (77, 40, "bf16"), (4737, 128, "bf16")])
+def test_router_logits_do_not_depend_on_the_tile(T, E, dtype):
+    """The tile is chosen by the token count; a token's logits must have the same bits in every one of them, so rows
+    routed alone (T = 32) equal the same rows among many."""
+    from kanjoos_b200 import ops
+    wr, _ = synth.router_weight(60, n_experts=E)
+    x = dev(synth.hidden_rows(60, T))
+    x = x.to(torch.bfloat16) if dtype == "bf16" else x
+    logits, pe, pw = ops.router_topk(x, bf16_dev(wr), 8)
+    for t0 in sorted({0, max(0, (T // 2) & ~1) if T >= 96 else 0, T - 32}):
+        lg, p, w = ops.router_topk(x[t0:t0 + 32].contiguous(), bf16_dev(wr), 8)
+        assert torch.equal(lg, logits[t0:t0 + 32])
+        assert torch.equal(p, pe.view(T, 8)[t0:t0 + 32].reshape(-1)) and torch.equal(w, pw.view(T, 8)[t0:t0 + 32].reshape(-1))
+    want = x.double() @ bf16_dev(wr).double().T
+    # f32 sums of 2048 exact products: the error of a sum is below sqrt(2048) * 2^-24 of its terms' 2-norm, 3e-6
+    assert report(logits.cpu().numpy(), want.float().cpu().numpy(), f"router logits {T}x{E}")["rel_rmse"] <= 1e-5
