@@ -76,6 +76,10 @@ inline cudaError_t launch_chain(void (*kern)(KArgs...), dim3 grid, dim3 block, s
 int make_row_tensor_map(CUtensorMap *map, const void *base, uint64_t rows, uint32_t row_bytes, uint32_t box_bytes,
                         uint32_t box_rows);
 
+// TMA descriptor for tile::gather4 copies out of a matrix of `rows` fp16 rows (`row_bytes` each, a multiple of 128,
+// base 16-byte aligned): one copy moves four rows of 64 elements into 512 bytes of a 128-byte-swizzled tile.
+int make_gather_tensor_map(CUtensorMap *map, const void *base, uint64_t rows, uint32_t row_bytes);
+
 // Limit (SM clock cycles) of the bounded waits of the decode-class kernels, as set by knj_decode_wait_limit.
 long long decode_wait_cycles();
 

@@ -8,22 +8,23 @@
 // one (expert, 128-row tile, token bucket); where a bucket has an even number of
 // row tiles, CTAs 2i and 2i+1 form a cluster and share one cta_group::2 MMA
 // (M = 256 over the pair, each CTA gathers half of the bucket's token rows):
-//   warps 0..7  unpackers: 2-D TMA boxes (32 rows x 144 B) bring the raw
-//               superblocks into a double-buffered staging area; per superblock
-//               the eight (d*sc, -dmin*m) pairs are formed in fp16 (exact), per
-//               slab each thread turns 16 code bytes into 32 fp16 weights and
-//               stores them into the K-major 128-byte-swizzled operand tile
-//               (three operand stages);
-//   warp 8      one elected thread issues tcgen05.mma (kind::f16) over the four
+//   warps 0..15 unpackers: per superblock the eight (d*sc, -dmin*m) pairs of a
+//               weight row are formed in fp16 (exact), per slab each thread turns
+//               16 code bytes of one matrix into 32 fp16 weights and stores them
+//               into the K-major 128-byte-swizzled operand tile or, for a bucket
+//               of up to 128 tokens, into the half of tensor memory that its
+//               accumulators leave free;
+//   warp 16     one elected thread issues tcgen05.mma (kind::f16) over the four
 //               16-wide steps of a slab and commits the stage back to the
 //               producers; in a pair the even CTA issues for both and its commit
 //               arrives on the barriers of both CTAs (tcgen05.commit with the
 //               multicast::cluster qualifier: a barrier arrival, no data moves);
-//   warps 9..12 loaders: gather the token rows of the slab with 16-byte cp.async
-//               straight into the swizzled tile; completion arrives on the stage
-//               barrier (cp.async.mbarrier.arrive.noinc), so several slabs are in
-//               flight with no registers held;
-//   warps 0..7  epilogue: tcgen05.ld of the accumulators (lane = weight row,
+//   warp 17     raw weights: one TMA box (128 rows x 144 B) per matrix and
+//               superblock into a ring of two to four buffers;
+//   warps 18..21 token rows: tile::gather4 TMA copies, four gathered rows of
+//               128 bytes each, into the swizzled tile; in a pair both CTAs'
+//               copies count on the even CTA's barrier;
+//   warps 0..15 epilogue: tcgen05.ld of the accumulators (lane = weight row,
 //               column = token), SiLU(gate)*up or the plain projection (or the
 //               weighted reduction into the token's sum), transposed through the
 //               idle operand stages, 16-byte row stores.
@@ -42,6 +43,8 @@
 #include "knj_common.cuh"
 #include "knj_q4k.h"
 
+#include <type_traits>
+
 using namespace knj;
 
 namespace {
@@ -49,9 +52,12 @@ namespace {
 constexpr int kRowsM = 128;        // weight rows per tile and CTA (MMA M per CTA)
 constexpr int kMaxTok = 256;       // token bucket (MMA N upper bound)
 constexpr int kSlabK = 64;         // K elements per pipeline stage (one 128-byte swizzle row)
-constexpr int kProducerThreads = 256;  // unpacker warps 0..7
-constexpr int kLoaderThreads = 128;    // loader warps 9..12
-constexpr int kThreads = kProducerThreads + 32 + kLoaderThreads;
+constexpr int kUnpackWarps = 16, kMmaWarp = 16, kRawWarp = 17, kRowsWarp = 18, kRowsWarps = 4;
+constexpr int kThreads = 32 * (kRowsWarp + kRowsWarps);
+constexpr int kSmallTok = 128;     // buckets up to this keep the unpacked weights in tensor memory
+constexpr int kStagesTmem = 4;     // operand stages of that form
+constexpr int kMaxStages = 4;
+constexpr int kMaxRaw = 4;         // raw-superblock buffers (as many as the bucket's token rows leave room for)
 constexpr float kActPrescale = 0.015625f;  // 2^-6
 
 struct TcParams {
@@ -75,7 +81,8 @@ struct TcParams {
   unsigned long long *trace;  // measurement builds: SM-clock stamps of CTA 0's first slabs
   int trace_ctas;             // per-CTA records that fit behind the 64 slab stamps
 #endif
-  CUtensorMap map0, map1;     // TMA descriptors of W0 / W1, box = one superblock (36 words) x 32 rows
+  CUtensorMap map0, map1;     // TMA descriptors of W0 / W1, box = one superblock (36 words) x 128 rows
+  CUtensorMap mapx;           // of X, for tile::gather4: one row of 64 fp16, 128-byte swizzle
 };
 
 #ifdef KNJ_TRACE
@@ -140,13 +147,20 @@ __device__ __forceinline__ uint32_t cluster_addr(const void *smem_ptr, uint32_t 
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_addr) : "memory");
 }
-// 16-byte asynchronous copy global -> shared (L2 only); src_bytes = 0 writes zeros
-__device__ __forceinline__ void cp_async16(void *dst_smem, const void *src, uint32_t src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst_smem)), "l"(src), "r"(src_bytes) : "memory");
-}
-// one arrival on the barrier once every cp.async this thread has issued so far has landed
-__device__ __forceinline__ void cp_async_arrive(uint64_t *bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+// four rows of 64 fp16 (x = first column), gathered by row index into 512 bytes of this CTA's swizzled tile; the
+// bytes count on the barrier at `bar_addr`, which in a pair may be the peer's
+template <int CG>
+__device__ __forceinline__ void tma_gather4(uint32_t dst_smem, const CUtensorMap *map, int x, const int4 &r, uint32_t bar_addr) {
+  if (CG == 1)
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+        ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w), "r"(bar_addr)
+        : "memory");
+  else
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+        ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w), "r"(bar_addr)
+        : "memory");
 }
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
@@ -187,6 +201,33 @@ __device__ __forceinline__ bool elect_one() {
 }
 // warp of the CTA, known to the compiler to be the same in all its lanes
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+// D(tmem) (+)= A(tmem) * B(smem desc): the weight operand read from tensor memory, K pairs along the columns
+template <int CG>
+__device__ __forceinline__ void tc_mma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  const uint32_t zero = 0;
+  if (CG == 1)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(zero), "r"(zero), "r"(zero), "r"(zero)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8, %9, %10, %11, %12}, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(zero), "r"(zero), "r"(zero), "r"(zero),
+          "r"(zero), "r"(zero), "r"(zero), "r"(zero)
+        : "memory");
+}
+// eight 32-bit columns of this thread's TMEM lane
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // 16 consecutive f32 columns of this thread's TMEM lane
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   uint32_t r[16];
@@ -213,9 +254,6 @@ __device__ __forceinline__ uint32_t instr_desc_f16(int m, int n) {
   return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-// the two unpacker warps that own the same 32 weight rows (one per 16-byte half) meet on their own barrier
-__device__ __forceinline__ void pair_sync(int pair) { asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory"); }
-
 constexpr int kQ6MaxSb = 4;  // Q6_K form: superblocks per weight row that the whole-tile staging holds (K <= 1024)
 
 template <int NMAT, int CG, int FMT = 0>
@@ -225,9 +263,10 @@ struct Smem {
   static constexpr int kStagesA = kStages, kStagesB = kStages;
   static constexpr int kTokCta = kMaxTok / CG;   // token rows this CTA stages per slab
   static constexpr int kATile = kRowsM * 128;    // 16 KB per matrix per stage
-  static constexpr int kBTile = kTokCta * 128;   // 32 KB (16 KB in a pair) per stage
-  // raw weights: Q4_K two buffers of one superblock per row; Q6_K the tile's rows whole, once (its 210-byte
-  // superblocks cannot be fetched as boxes: rows are only 2-byte aligned)
+  static constexpr int kBTile = kTokCta * 128;   // 32 KB (16 KB in a pair) per stage, less for a smaller bucket
+  // raw weights: Q4_K a ring of buffers of one superblock per row, two behind a full bucket's token stages, more
+  // behind a smaller one's (the ring starts where the bucket's token rows end); Q6_K the tile's rows whole, once
+  // (its 210-byte superblocks cannot be fetched as boxes: rows are only 2-byte aligned)
   static constexpr int kRawBuf = FMT == 1 ? kRowsM * kQ6MaxSb * KNJ_Q6K_BYTES : NMAT * kRowsM * KNJ_Q4K_BYTES;
   static constexpr int kOffA = 0;
   static constexpr int kOffB = kOffA + kStagesA * NMAT * kATile;
@@ -337,29 +376,41 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
   const int nsb = p.K / KNJ_QK_K, nslab = p.K / kSlabK;
 
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + S::kOffBars);
-  uint64_t *full = bars;                           // [kStages] unpackers + loaders -> MMA (the even CTA's are used)
-  uint64_t *empty = full + kStages;                // [kStages] MMA -> unpackers and loaders
-  uint64_t *locB = empty + kStages;                // [kStages] odd CTA only: its own loaders' copies landed
-  uint64_t *raw_full = locB + kStages;             // [2 buffers][4 row groups] TMA boxes landed
-  uint64_t *acc_full = raw_full + 8;
+  uint64_t *full = bars;                           // [kMaxStages] unpackers + row copies -> MMA (the even CTA's are used)
+  uint64_t *empty = full + kMaxStages;             // [kMaxStages] MMA -> unpackers and row copies
+  uint64_t *raw_full = empty + kMaxStages;         // [kMaxRaw] TMA boxes landed (Q6_K: one per 32-row group)
+  uint64_t *raw_empty = raw_full + kMaxRaw;        // [kMaxRaw] unpackers are done with the buffer
+  uint64_t *acc_full = raw_empty + kMaxRaw;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
   volatile int *s_fail = reinterpret_cast<volatile int *>(tmem_slot + 1);  // raised by the first wait that gives up
   int32_t *s_pair = reinterpret_cast<int32_t *>(smem + S::kOffPairs);
   int32_t *s_row = reinterpret_cast<int32_t *>(smem + S::kOffRows);
 
-  if (tid == 0) {
-    // one "full" barrier per stage: 8 unpacker warps per CTA, this CTA's loader threads (asynchronous-copy
-    // arrivals) and, in a pair, one relayed arrival for the odd CTA's loaders
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(&full[s], CG * 8 + kLoaderThreads + (CG == 2 ? 1 : 0));
-      mbar_init(&empty[s], 1);
-      mbar_init(&locB[s], kLoaderThreads);
+  // Up to 128 tokens the accumulators leave half of tensor memory free: the unpacked weights go there (tcgen05.st, four
+  // stages of 32 columns per matrix) and the MMA reads its A operand from tensor memory. Stored to shared memory they
+  // cross its 128 B/cycle pipe twice. With sixteen unpacker warps and gathered rows, gate+up takes 112 us at 100 tokens and
+  // 88 us at 512 Zipf-routed ones, against 133 and 104 with eight warps, cp.async rows and A in shared memory. Above 128
+  // tokens two accumulators of 256 columns fill tensor memory (full buckets: 828 -> 743 us at 16384 tokens).
+  const bool a_tmem = n_mma <= kSmallTok;
+  const int n_stages = a_tmem ? kStagesTmem : kStages;
+  const int b_tile = n_cta * 128;                                   // a multiple of 1024: n_cta is one of 8
+  const int off_b = a_tmem ? 0 : S::kOffB;
+  const int off_raw = FMT == 1 ? S::kOffRaw : off_b + n_stages * b_tile;
+  const int n_raw = min(kMaxRaw, (S::kOffPairs - off_raw) / S::kRawBuf);  // Q4_K: two at 256 tokens, up to four below
+  auto issue_raw = [&](int b, int buf) {
+    mbar_expect_tx(&raw_full[buf], (uint32_t)S::kRawBuf);
+#pragma unroll
+    for (int mat = 0; mat < NMAT; ++mat)
+      tma_load_rows(smem + off_raw + buf * S::kRawBuf + mat * kRowsM * KNJ_Q4K_BYTES, (GATEUP && mat == 1) ? &p.map1 : &p.map0,
+                    b * (KNJ_Q4K_BYTES / 4), e * p.N + m0 + (GATEUP ? 0 : mat * kRowsM), &raw_full[buf]);
+  };
+  if (warp == kRawWarp && elect_one()) {
+    // the weights depend on nothing in this launch: the first superblocks travel while the rest of the prologue runs
+    for (int i = 0; i < kMaxRaw; ++i) {
+      mbar_init(&raw_full[i], 1);
+      mbar_init(&raw_empty[i], kUnpackWarps);
     }
-    for (int i = 0; i < 8; ++i) mbar_init(&raw_full[i], 1);
-    mbar_init(acc_full, 1);
-    *s_fail = 0;
-    if (CG == 2) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    else mbar_init_fence();
+    mbar_init_fence();
     if (FMT == 1) {
       // Q6_K: the tile's 128 rows are contiguous in HBM and start on a 16-byte boundary (tiles start at multiples
       // of 128 rows, 32 rows are a multiple of 16 bytes): four bulk copies, one per 32-row group, each on its own
@@ -371,10 +422,26 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
         mbar_expect_tx(&raw_full[g], grp);
         bulk_g2s(smem + S::kOffRaw + g * grp, src + (size_t)g * grp, grp, &raw_full[g]);
       }
+    } else {
+      for (int b = 0; b < nsb && b < n_raw; ++b) issue_raw(b, b);
     }
   }
-  for (int i = tid; i < kMaxTok; i += kThreads) {
-    int pr = -1, rw = -1;
+  if (tid == 0) {
+    // one "full" barrier per stage: 16 unpacker warps per CTA and the even CTA's first row warp, which also announces
+    // the bytes of both CTAs' token rows
+    for (int s = 0; s < kMaxStages; ++s) {
+      mbar_init(&full[s], CG * kUnpackWarps + 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(acc_full, 1);
+    *s_fail = 0;
+    mbar_init_fence();
+  }
+  for (int i = tid; i < n_mma; i += kThreads) {
+    int pr = -1;
+    // the tokens that pad the bucket to a multiple of 16 read the bucket's first row; their columns are never stored
+    int rw = p.pair_idx[(size_t)e * p.idxStride + tok0];
+    rw = p.row_map ? p.row_map[rw] : rw / p.row_div;
     if (i < ntok) {
       pr = p.pair_idx[(size_t)e * p.idxStride + tok0 + i];
       rw = p.row_map ? p.row_map[pr] : pr / p.row_div;
@@ -383,7 +450,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
     s_row[i] = rw;
   }
   constexpr uint32_t kTmemCols = NMAT == 2 ? 512 : 256;
-  if (warp == 8) {
+  if (warp == kMmaWarp) {
     tmem_alloc<CG>(tmem_slot, kTmemCols);
     tmem_relinquish<CG>();
   }
@@ -392,98 +459,107 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
   if (CG == 2) cluster_sync_all();  // the peer's barriers are initialised before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  const int d_cols = a_tmem ? kSmallTok : kMaxTok;                    // accumulator columns per matrix
+  const uint32_t a_base = tmem_base + kTmemCols / 2;                   // a_tmem: weight stages of 32 columns per matrix
   bool ok = true;  // once false this thread skips all work and waits but still meets every barrier
+  // 16 weights of a row, K = 8 * c0 + [0, 16) of the slab: eight columns of the lane, or two chunks of the swizzled row
+  auto store_weights = [&](auto ta, const uint32_t (&o)[8], int stage, int mat, int row, int c0) {
+    if constexpr (decltype(ta)::value) {
+      tmem_st8(a_base + ((uint32_t)(row & 96) << 16) + (stage * NMAT + mat) * 32 + 4 * c0, o);
+    } else {
+      uint8_t *at = smem + S::kOffA + (stage * NMAT + mat) * S::kATile + row * 128;
+      *reinterpret_cast<uint4 *>(at + (((c0) ^ (row & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+      *reinterpret_cast<uint4 *>(at + (((c0 + 1) ^ (row & 7)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+    }
+  };
+  auto publish = [&](auto ta, int stage) {  // the warp's part of the stage is written
+    if constexpr (decltype(ta)::value) {
+      tmem_st_wait();
+      tc_fence_before();
+    } else {
+      fence_proxy_async();
+    }
+    __syncwarp();
+    if (lane == 0) {
+      if (CG == 2) mbar_arrive_cluster(cluster_addr(&full[stage], 0));
+      else mbar_arrive(&full[stage]);
+    }
+  };
+  // a warp goes on or gives up as a whole: its accesses to tensor memory are warp-wide
+  auto wait_all = [&](uint64_t *bar, uint32_t parity) {
+    if (ok && !mbar_wait(bar, parity, s_fail)) ok = false;
+    ok = __all_sync(0xffffffffu, ok);
+    return ok;
+  };
 
-  if (FMT == 1 && warp < 8) {
+  if (FMT == 1 && warp < kUnpackWarps) {
     // =========================== producers, Q6_K ===========================
-    const int row = tid & 127, half = tid >> 7;  // weight row, which 16 of a quadrant's 32 weights
+    // weight row, which 16 of a quadrant's 32 weights, which of the slab's two quadrants
+    const int row = tid & 127, half = (tid >> 7) & 1, par = tid >> 8;
     const int row_bytes = nsb * KNJ_Q6K_BYTES;
     uint8_t *rawq = smem + S::kOffRaw;
-    if (!mbar_wait(&raw_full[warp & 3], 0, s_fail)) ok = false;  // this warp's 32 rows have landed
+    wait_all(&raw_full[warp & 3], 0);  // this warp's 32 rows have landed
     const uint8_t *rrow = rawq + (size_t)row * row_bytes;
     const __half2 k1056 = __float2half2_rn(1056.0f);  // 1024 (the byte-to-fp16 trick) + 32 (the code's offset)
+    auto unpack = [&](auto ta) {
+    int stage = 0;
+    uint32_t empty_par = 1;  // a fresh barrier passes a wait for parity 1
     for (int ks = 0; ks < nslab; ++ks) {
-      if (*s_fail) ok = false;
-      if (!ok) break;
-      const int stage = ks % kStages;
-      if (ks >= kStages && !mbar_wait(&empty[stage], ((ks / kStages) - 1) & 1, s_fail)) { ok = false; break; }
+      if (!wait_all(&empty[stage], empty_par)) break;
       tc_fence_after();
       const int sl = ks & 3, hf = sl >> 1;
       const uint8_t *blk = rrow + (ks >> 2) * KNJ_Q6K_BYTES;
       const float d = __half2float(__ushort_as_half(*reinterpret_cast<const uint16_t *>(blk + 208)));
       uint32_t qh[4];
       lds16_u16(blk + 128 + 32 * hf + 16 * half, qh);
-      uint8_t *at = smem + S::kOffA + stage * S::kATile + row * 128;
+      const int c = 2 * (sl & 1) + par;  // quadrant of the 128-weight half: weights 32 c + l, l = 16 half + [0, 16)
+      uint32_t ql[4];
+      lds16_u16(blk + 64 * hf + 32 * par + 16 * half, ql);
+      const float sc = (float)reinterpret_cast<const int8_t *>(blk)[192 + 8 * hf + half + 2 * c];
+      const __half2 ds = __float2half2_rn(d * sc);
+      uint32_t o[8];
 #pragma unroll
-      for (int par = 0; par < 2; ++par) {
-        const int c = 2 * (sl & 1) + par;  // quadrant of the 128-weight half: weights 32 c + l, l = 16 half + [0, 16)
-        uint32_t ql[4];
-        lds16_u16(blk + 64 * hf + 32 * par + 16 * half, ql);
-        const float sc = (float)reinterpret_cast<const int8_t *>(blk)[192 + 8 * hf + half + 2 * c];
-        const __half2 ds = __float2half2_rn(d * sc);
-        uint32_t o[8];
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-          const uint32_t nib = ((sl & 1) ? (ql[w] >> 4) : ql[w]) & 0x0f0f0f0fu;
-          const uint32_t q4 = nib | (((qh[w] >> (2 * c)) & 0x03030303u) << 4);
-          const uint32_t e01 = __byte_perm(q4, 0x64646464u, 0x4140);
-          const uint32_t e23 = __byte_perm(q4, 0x64646464u, 0x4342);
-          const __half2 h01 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&e01), k1056), ds);
-          const __half2 h23 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&e23), k1056), ds);
-          o[2 * w] = *reinterpret_cast<const uint32_t *>(&h01);
-          o[2 * w + 1] = *reinterpret_cast<const uint32_t *>(&h23);
-        }
-        const int c0 = 4 * par + 2 * half;
-        *reinterpret_cast<uint4 *>(at + (((c0) ^ (row & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-        *reinterpret_cast<uint4 *>(at + (((c0 + 1) ^ (row & 7)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+      for (int w = 0; w < 4; ++w) {
+        const uint32_t nib = ((sl & 1) ? (ql[w] >> 4) : ql[w]) & 0x0f0f0f0fu;
+        const uint32_t q4 = nib | (((qh[w] >> (2 * c)) & 0x03030303u) << 4);
+        const uint32_t e01 = __byte_perm(q4, 0x64646464u, 0x4140);
+        const uint32_t e23 = __byte_perm(q4, 0x64646464u, 0x4342);
+        const __half2 h01 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&e01), k1056), ds);
+        const __half2 h23 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&e23), k1056), ds);
+        o[2 * w] = *reinterpret_cast<const uint32_t *>(&h01);
+        o[2 * w + 1] = *reinterpret_cast<const uint32_t *>(&h23);
       }
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) {
-        if (CG == 2) mbar_arrive_cluster(cluster_addr(&full[stage], 0));
-        else mbar_arrive(&full[stage]);
-      }
+      store_weights(ta, o, stage, 0, row, 4 * par + 2 * half);
+      publish(ta, stage);
+      if (++stage == n_stages) { stage = 0; empty_par ^= 1u; }
     }
-  } else if (warp < 8) {
-    // =========================== producers ===========================
-    const int row = tid & 127, half = tid >> 7;  // weight row, which 16 of the slab's 32 code bytes
-    const int pair = warp & 3;                   // rows 32*pair .. 32*pair+31: this warp and warp ^ 4
-    // one TMA box per matrix and row group: 32 rows x one superblock (a single copy instruction each; per-row
-    // bulk copies cost the copy unit about 25 cycles apiece and stalled every superblock boundary)
-    auto issue_raw = [&](int b) {
-      if (warp < 4 && lane == 0) {
-        uint64_t *bar = &raw_full[(b & 1) * 4 + pair];
-        mbar_expect_tx(bar, (uint32_t)NMAT * 32u * KNJ_Q4K_BYTES);
-#pragma unroll
-        for (int mat = 0; mat < NMAT; ++mat) {
-          uint8_t *dst = smem + S::kOffRaw + (b & 1) * S::kRawBuf + (mat * kRowsM + 32 * pair) * KNJ_Q4K_BYTES;
-          const int y = e * p.N + m0 + (GATEUP ? 0 : mat * kRowsM) + 32 * pair;
-          tma_load_rows(dst, (GATEUP && mat == 1) ? &p.map1 : &p.map0, b * (KNJ_Q4K_BYTES / 4), y, bar);
-        }
-      }
     };
-    fence_proxy_async();
-    issue_raw(0);
-    for (int b = 0; b < nsb; ++b) {
-      // both warps of the row group are done reading the buffer the next superblock lands in
-      pair_sync(pair);
-      if (*s_fail) ok = false;
-      if (!ok) continue;
-      if (b + 1 < nsb) {
-        fence_proxy_async();
-        issue_raw(b + 1);
-      }
-      if (!mbar_wait(&raw_full[(b & 1) * 4 + pair], (b >> 1) & 1, s_fail)) { ok = false; continue; }
-      const uint8_t *raw = smem + S::kOffRaw + (b & 1) * S::kRawBuf;
+    if (a_tmem) unpack(std::true_type{});
+    else unpack(std::false_type{});
+  } else if (warp < kUnpackWarps) {
+    // =========================== producers ===========================
+    // Two matrices: 256 threads each, a thread takes 16 of the slab's 32 code bytes of its row. One matrix: a thread
+    // takes the low or the high nibbles of its 16 bytes.
+    constexpr int kPar = NMAT;                       // nibble planes per thread
+    const int row = tid & 127, half = (tid >> 7) & 1;
+    const int mat = NMAT == 2 ? tid >> 8 : 0, par0 = NMAT == 2 ? 0 : tid >> 8;
+    auto unpack = [&](auto ta) {
+    // few tokens: the unpackers set the pace, so the weights are formed before the stage is waited for; full buckets
+    // wait for the tensor pipe, and holding formed weights back there was slower (1.96 against 1.89 ms at 16384 tokens)
+    constexpr bool kEarly = decltype(ta)::value;
+    int buf = 0, stage = 0;
+    uint32_t raw_par = 0, empty_par = 1;             // a fresh barrier passes a wait for parity 1
+    for (int b = 0; b < nsb && ok; ++b) {
+      if (!wait_all(&raw_full[buf], raw_par)) break;
+      const uint8_t *raw = smem + off_raw + buf * S::kRawBuf + (mat * kRowsM + row) * KNJ_Q4K_BYTES;
 
       // ---- once per superblock: (d*sc, -dmin*m) of this row's eight sub-blocks in fp16.
       // d*sc is an 11-bit by 6-bit product, so one fp16 multiply rounds it exactly as a
       // float multiply followed by a conversion would.
       const __half2 k1024 = __float2half2_rn(1024.0f);
-      __half2 d1h[NMAT][8], m1h[NMAT][8];
-#pragma unroll
-      for (int mat = 0; mat < NMAT; ++mat) {
-        const uint4 hdr = *reinterpret_cast<const uint4 *>(raw + (mat * kRowsM + row) * KNJ_Q4K_BYTES);
+      __half2 d1h[4 * kPar], m1h[4 * kPar];
+      {
+        const uint4 hdr = *reinterpret_cast<const uint4 *>(raw);
         const __half2 dd = __half2half2(__ushort_as_half((unsigned short)(hdr.x & 0xffffu)));
         const __half2 dm = __hneg2(__half2half2(__ushort_as_half((unsigned short)(hdr.x >> 16))));
         const uint32_t sc4[2] = {hdr.y & 0x3f3f3f3fu, (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u)};
@@ -497,130 +573,149 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
             const uint32_t em = __byte_perm(mn4[hb], 0x64646464u, pr ? 0x4342 : 0x4140);
             const __half2 s2 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&es), k1024), dd);
             const __half2 m2 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&em), k1024), dm);
-            d1h[mat][4 * hb + 2 * pr] = __low2half2(s2);
-            d1h[mat][4 * hb + 2 * pr + 1] = __high2half2(s2);
-            m1h[mat][4 * hb + 2 * pr] = __low2half2(m2);
-            m1h[mat][4 * hb + 2 * pr + 1] = __high2half2(m2);
+            const int G = 2 * hb + pr;
+            if (kPar == 2) {
+              d1h[2 * G] = __low2half2(s2);
+              d1h[2 * G + 1] = __high2half2(s2);
+              m1h[2 * G] = __low2half2(m2);
+              m1h[2 * G + 1] = __high2half2(m2);
+            } else {
+              d1h[G] = par0 ? __high2half2(s2) : __low2half2(s2);
+              m1h[G] = par0 ? __high2half2(m2) : __low2half2(m2);
+            }
           }
         }
       }
 
 #pragma unroll
       for (int G = 0; G < 4; ++G) {
-        if (!ok) break;
-        const int ks = b * 4 + G, stage = ks % kStages;
+        [[maybe_unused]] const int ks = b * 4 + G;
         KNJ_TC_STAMP(blockIdx.x == 0 && tid == 0 && ks < 12, 4 * ks + 0);
-        if (ks >= kStages && !mbar_wait(&empty[stage], ((ks / kStages) - 1) & 1, s_fail)) { ok = false; break; }
-        tc_fence_after();
-        KNJ_TC_STAMP(blockIdx.x == 0 && tid == 0 && ks < 12, 4 * ks + 1);
-        // ---- weight operand(s): 16 code bytes -> 16 low-nibble + 16 high-nibble weights of this row
+        // the codes are read before the stage is waited for; after the last ones the raw buffer goes back
+        const uint4 q = *reinterpret_cast<const uint4 *>(raw + KNJ_Q4K_OFF_QS + 32 * G + 16 * half);
+        if (G == 3) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&raw_empty[buf]);
+        }
+        if (!kEarly && !wait_all(&empty[stage], empty_par)) break;
+        // ---- weight operand: 16 code bytes -> 16 low-nibble and / or 16 high-nibble weights of this row
+        const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
+        uint32_t o[kPar][8];
 #pragma unroll
-        for (int mat = 0; mat < NMAT; ++mat) {
-          const uint4 q = *reinterpret_cast<const uint4 *>(raw + (mat * kRowsM + row) * KNJ_Q4K_BYTES + KNJ_Q4K_OFF_QS + 32 * G + 16 * half);
-          uint8_t *at = smem + S::kOffA + (stage * NMAT + mat) * S::kATile + row * 128;
-          const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
+        for (int j = 0; j < kPar; ++j) {
+          const __half2 d1 = d1h[kPar * G + j], m1 = m1h[kPar * G + j];
 #pragma unroll
-          for (int par = 0; par < 2; ++par) {
-            const __half2 d1 = d1h[mat][2 * G + par], m1 = m1h[mat][2 * G + par];
-            uint32_t o[8];
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-              // the four codes of this word as bytes, then pairs (k0,k1), (k2,k3) as fp16 1024+q
-              const uint32_t nib = (par ? (qw[w] >> 4) : qw[w]) & 0x0f0f0f0fu;
-              const uint32_t e01 = __byte_perm(nib, 0x64646464u, 0x4140);
-              const uint32_t e23 = __byte_perm(nib, 0x64646464u, 0x4342);
-              const __half2 h01 = __hfma2(__hsub2(*reinterpret_cast<const __half2 *>(&e01), k1024), d1, m1);
-              const __half2 h23 = __hfma2(__hsub2(*reinterpret_cast<const __half2 *>(&e23), k1024), d1, m1);
-              o[2 * w] = *reinterpret_cast<const uint32_t *>(&h01);
-              o[2 * w + 1] = *reinterpret_cast<const uint32_t *>(&h23);
-            }
-            // 16 weights = two 16-byte chunks: k_local = 32*par + 16*half + [0,16)
-            const int c0 = 4 * par + 2 * half;
-            *reinterpret_cast<uint4 *>(at + (((c0) ^ (row & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-            *reinterpret_cast<uint4 *>(at + (((c0 + 1) ^ (row & 7)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+          for (int w = 0; w < 4; ++w) {
+            // the four codes of this word as bytes, then pairs (k0,k1), (k2,k3) as fp16 1024+q
+            const uint32_t nib = (qw[w] >> (4 * (par0 + j))) & 0x0f0f0f0fu;
+            const uint32_t e01 = __byte_perm(nib, 0x64646464u, 0x4140);
+            const uint32_t e23 = __byte_perm(nib, 0x64646464u, 0x4342);
+            const __half2 h01 = __hfma2(__hsub2(*reinterpret_cast<const __half2 *>(&e01), k1024), d1, m1);
+            const __half2 h23 = __hfma2(__hsub2(*reinterpret_cast<const __half2 *>(&e23), k1024), d1, m1);
+            o[j][2 * w] = *reinterpret_cast<const uint32_t *>(&h01);
+            o[j][2 * w + 1] = *reinterpret_cast<const uint32_t *>(&h23);
           }
         }
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) {
-          if (CG == 2) mbar_arrive_cluster(cluster_addr(&full[stage], 0));
-          else mbar_arrive(&full[stage]);
-        }
+        if (kEarly && !wait_all(&empty[stage], empty_par)) break;
+        KNJ_TC_STAMP(blockIdx.x == 0 && tid == 0 && ks < 12, 4 * ks + 1);
+        tc_fence_after();
+        // 16 weights per plane: k_local = 32*par + 16*half + [0,16)
+#pragma unroll
+        for (int j = 0; j < kPar; ++j) store_weights(ta, o[j], stage, mat, row, 4 * (par0 + j) + 2 * half);
+        publish(ta, stage);
         KNJ_TC_STAMP(blockIdx.x == 0 && tid == 0 && ks < 12, 4 * ks + 2);
+        if (++stage == n_stages) { stage = 0; empty_par ^= 1u; }
+      }
+      if (++buf == n_raw) { buf = 0; raw_par ^= 1u; }
+    }
+    };
+    if (a_tmem) unpack(std::true_type{});
+    else unpack(std::false_type{});
+  } else if (warp == kRawWarp) {
+    // =========================== raw weights ===========================
+    if (FMT == 0 && elect_one()) {
+      int buf = 0;
+      uint32_t par = 0;
+      for (int b = n_raw; b < nsb; ++b) {
+        if (!mbar_wait(&raw_empty[buf], par, s_fail)) { ok = false; break; }
+        fence_proxy_async();  // the buffer was read through the generic proxy
+        issue_raw(b, buf);
+        if (++buf == n_raw) { buf = 0; par ^= 1u; }
       }
     }
-  } else if (warp >= 9) {
-    // =========================== loaders ===========================
-    // rows of 64 fp16 per slab; 16-byte chunk c of row r lands at chunk c ^ (r & 7). Asynchronous copies:
-    // nothing waits for the gathered rows in registers, so as many slabs travel as there are stages, and
-    // the stage's barrier gets this thread's arrival when its copies have landed. (A register path would
-    // stall on the release fence of every hand-off until its prefetched loads return.) In a pair each CTA
-    // gathers half of the bucket's rows.
-    constexpr int kRpt = S::kTokCta / 16;  // rows per thread and slab
-    const int lt = tid - (kProducerThreads + 32);
-    const int c = lt & 7, r0 = lt >> 3;  // 16 rows per pass
-    const __half *rowp[kRpt];
+  } else if (warp >= kRowsWarp) {
+    // =========================== token rows ===========================
+    // One elected thread in each of four warps gathers four rows a copy; the even CTA's first one announces the bytes of
+    // both CTAs. 16-byte cp.async by 128 threads, the form before, took 1200 cycles to issue a full bucket's slab and
+    // ~1600 more to land, which with three stages bound the loop; one copy per lane of one warp took ~75 cycles a copy
+    // (the lanes' operands reach the copy unit one by one; 2400 us a step of 16384 tokens).
+    const int w0 = warp - kRowsWarp;
+    if (4 * w0 < n_cta && elect_one()) {
+      constexpr int kQuads = S::kTokCta / (4 * kRowsWarps);
+      int4 rows[kQuads];  // in registers: read from shared memory at each copy, a step of 16384 tokens took 1970 us, not 1863
 #pragma unroll
-    for (int j = 0; j < kRpt; ++j) {
-      const int r = r0 + 16 * j;
-      const int xr = r < n_cta ? s_row[rank * n_cta + r] : -1;
-      rowp[j] = xr >= 0 ? p.X + (size_t)xr * p.K + c * 8 : nullptr;
-    }
-    for (int ks = 0; ks < nslab && ok; ++ks) {  // loaders meet no CTA barrier before the final one
-      const int stage = ks % kStages;
-      [[maybe_unused]] const bool ltr = blockIdx.x == 0 && lt == 0 && ks < 12;
-      KNJ_TC_STAMP(ltr, 64 + 4 * ks);
-      if (ks >= kStages && !mbar_wait(&empty[stage], ((ks / kStages) - 1) & 1, s_fail)) { ok = false; break; }
-      KNJ_TC_STAMP(ltr, 64 + 4 * ks + 1);
-      uint8_t *bt = smem + S::kOffB + stage * S::kBTile;
-#pragma unroll
-      for (int j = 0; j < kRpt; ++j) {
-        const int r = r0 + 16 * j;
-        if (r < n_cta)
-          cp_async16(bt + r * 128 + ((c ^ (r & 7)) << 4), rowp[j] ? (const void *)(rowp[j] + ks * kSlabK) : (const void *)p.X,
-                     rowp[j] ? 16u : 0u);
+      for (int j = 0; j < kQuads; ++j) {
+        const int r = 4 * (w0 + kRowsWarps * j);
+        rows[j] = r < n_cta ? *reinterpret_cast<const int4 *>(s_row + rank * n_cta + r) : make_int4(0, 0, 0, 0);
       }
-      cp_async_arrive(rank == 0 ? &full[stage] : &locB[stage]);
-      KNJ_TC_STAMP(ltr, 64 + 4 * ks + 3);
+      int stage = 0;
+      uint32_t par = 1;  // a fresh barrier passes a wait for parity 1
+      for (int ks = 0; ks < nslab; ++ks) {
+        [[maybe_unused]] const bool ltr = blockIdx.x == 0 && w0 == 0 && ks < 12;
+        KNJ_TC_STAMP(ltr, 64 + 4 * ks);
+        if (!mbar_spin(&empty[stage], par, s_fail)) { ok = false; break; }
+        KNJ_TC_STAMP(ltr, 64 + 4 * ks + 1);
+        if (rank == 0 && w0 == 0) mbar_expect_tx(&full[stage], (uint32_t)n_mma * 128u);
+        const uint32_t bar = CG == 2 ? cluster_addr(&full[stage], 0) : smem_u32(&full[stage]);
+        const uint32_t dst = smem_u32(smem + off_b + stage * b_tile);
+#pragma unroll
+        for (int j = 0; j < kQuads; ++j) {
+          const int r = 4 * (w0 + kRowsWarps * j);
+          if (r < n_cta) tma_gather4<CG>(dst + r * 128, &p.mapx, ks * kSlabK, rows[j], bar);
+        }
+        KNJ_TC_STAMP(ltr, 64 + 4 * ks + 3);
+        if (++stage == n_stages) { stage = 0; par ^= 1u; }
+      }
     }
-  } else if (CG == 2 && rank == 1) {
-    // =========================== relay (odd CTA) ===========================
-    // cp.async completions can only arrive on a barrier of their own CTA: pass them on to the MMA thread
-    if (elect_one())
-    for (int ks = 0; ks < nslab && ok; ++ks) {
-      const int sb = ks % kStages;
-      if (!mbar_spin(&locB[sb], (ks / kStages) & 1, s_fail)) { ok = false; break; }
-      mbar_arrive_cluster(cluster_addr(&full[sb], 0));
-    }
-  } else if (elect_one()) {
+  } else if (rank == 0 && elect_one()) {
     // =========================== MMA issue ===========================
-    // One elected thread of warp 8. The branch has to be uniform up to elect.sync: picked by `lane == 0` instead, the
+    // One elected thread of warp 16. The branch has to be uniform up to elect.sync: picked by `lane == 0` instead, the
     // same loop took 93 cycles an instruction whatever N was (its operands then have to be moved to uniform registers
     // one instruction at a time), against N / 2 cycles, the tensor pipe's own rate, this way. Consecutive instructions
     // alternate between the two accumulators. One "full" barrier per stage covers both operands, one commit the CTA pair.
     const uint32_t idesc = instr_desc_f16(kRowsM * CG, n_mma);
-    const uint64_t a_desc0 = smem_desc_sw128(smem_u32(smem + S::kOffA)), b_desc0 = smem_desc_sw128(smem_u32(smem + S::kOffB));
+    const uint64_t a_desc0 = smem_desc_sw128(smem_u32(smem + S::kOffA)), b_desc0 = smem_desc_sw128(smem_u32(smem + off_b));
     int st = 0;
     uint32_t par = 0;
     for (int ks = 0; ks < nslab; ++ks) {
       if (!mbar_spin(&full[st], par, s_fail)) { ok = false; break; }
-      // No proxy fence here: the unpackers fence their own stores before arriving, the gathered rows are
-      // complete when their copies' arrivals are (the hand-off CUTLASS' cp.async tcgen05 main loop relies on),
-      // and a fence.proxy.async in this thread would wait for the shared-memory reads of every MMA in flight.
+      // No proxy fence here: the unpackers fence their own stores before arriving, the token rows come through the
+      // async proxy, and a fence.proxy.async in this thread would wait for the shared-memory reads of every MMA in flight.
       tc_fence_after();
       KNJ_TC_STAMP(blockIdx.x == 0 && ks < 12, 4 * ks + 3);
-      const uint64_t a_desc = a_desc0 + (uint32_t)(st * NMAT * S::kATile) / 16, b_desc = b_desc0 + (uint32_t)(st * S::kBTile) / 16;
+      const uint64_t a_desc = a_desc0 + (uint32_t)(st * NMAT * S::kATile) / 16, b_desc = b_desc0 + (uint32_t)(st * b_tile) / 16;
+      if (a_tmem) {
+        const uint32_t a_addr = a_base + st * NMAT * 32;
 #pragma unroll
-      for (int k = 0; k < kSlabK / 16; ++k) {
+        for (int k = 0; k < kSlabK / 16; ++k) {
 #pragma unroll
-        for (int mat = 0; mat < NMAT; ++mat)
-          tc_mma_f16<CG>(tmem_base + mat * kMaxTok, a_desc + (uint32_t)(mat * S::kATile + k * 32) / 16, b_desc + (uint32_t)(k * 32) / 16, idesc,
-                         (ks > 0 || k > 0) ? 1u : 0u);
+          for (int mat = 0; mat < NMAT; ++mat)
+            tc_mma_f16_ta<CG>(tmem_base + mat * kSmallTok, a_addr + mat * 32 + k * 8, b_desc + (uint32_t)(k * 32) / 16, idesc,
+                              (ks > 0 || k > 0) ? 1u : 0u);
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < kSlabK / 16; ++k) {
+#pragma unroll
+          for (int mat = 0; mat < NMAT; ++mat)
+            tc_mma_f16<CG>(tmem_base + mat * kMaxTok, a_desc + (uint32_t)(mat * S::kATile + k * 32) / 16, b_desc + (uint32_t)(k * 32) / 16, idesc,
+                           (ks > 0 || k > 0) ? 1u : 0u);
+        }
       }
       if (CG == 2) tc_commit_pair(smem_u32(&empty[st]));
       else tc_commit_addr<CG>(smem_u32(&empty[st]));
       KNJ_TC_STAMP(blockIdx.x == 0 && ks < 12, 128 + ks);
-      if (++st == kStages) { st = 0; par ^= 1u; }
+      if (++st == n_stages) { st = 0; par ^= 1u; }
     }
     if (ok) {
       if (CG == 2) tc_commit_pair(smem_u32(acc_full));
@@ -629,12 +724,10 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
   }
 
   // =========================== epilogue ===========================
-  if (warp != 8) {
-    // unpackers and loaders alike (12 warps); warp w may read the 32 TMEM lanes 32 * (w % 4)
-    constexpr int kEpiWarps = 12;
-    const int ew = warp < 8 ? warp : warp - 1;          // 0..11
-    const int slot = warp < 8 ? (warp >> 2) : 2;        // which of the three warps of a lane group
-    if (ok && !mbar_wait(acc_full, 0, s_fail)) ok = false;
+  if (warp < kUnpackWarps) {
+    // warp w may read the 32 TMEM lanes 32 * (w % 4)
+    const int slot = warp >> 2;        // which of the four warps of a lane group
+    wait_all(acc_full, 0);
     tc_fence_after();
     KNJ_TC_REC(1);
     // The accumulator rows are output indices (one per thread) and the columns tokens, while the outputs are
@@ -650,12 +743,12 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
 #pragma unroll 1
     for (int mat = 0; mat < kEpiMats; ++mat) {
       if (ok) {
-        for (int c = slot; c * 16 < n_mma; c += 3) {
+        for (int c = slot; c * 16 < n_mma; c += kUnpackWarps / 4) {
           float g[16];
-          tmem_ld16(tmem_base + ((uint32_t)lane_base << 16) + mat * kMaxTok + c * 16, g);
+          tmem_ld16(tmem_base + ((uint32_t)lane_base << 16) + mat * d_cols + c * 16, g);
           if (GATEUP) {
             float u[16];
-            tmem_ld16(tmem_base + ((uint32_t)lane_base << 16) + kMaxTok + c * 16, u);
+            tmem_ld16(tmem_base + ((uint32_t)lane_base << 16) + d_cols + c * 16, u);
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
               // fast division: the IEEE one takes its slow path whenever exp(-g) overflows
@@ -671,12 +764,12 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
         }
       }
       KNJ_TC_STAMP(tr, 49 + 2 * mat);
-      asm volatile("bar.sync 5, 384;" ::: "memory");
+      asm volatile("bar.sync 5, 512;" ::: "memory");
       if (ok) {
         constexpr int kLanesPerRow = kRowB / 16;            // 16 (fp16) or 32 (f32)
         constexpr int kRowsPerInstr = 32 / kLanesPerRow;    // 2 or 1
         const int sub = lane / kLanesPerRow, l16 = lane % kLanesPerRow;
-        for (int r = ew * kRowsPerInstr + sub; r < ntok; r += kEpiWarps * kRowsPerInstr) {
+        for (int r = warp * kRowsPerInstr + sub; r < ntok; r += kUnpackWarps * kRowsPerInstr) {
           const int pr = s_pair[r];
           const uint4 v = *reinterpret_cast<const uint4 *>(stg + r * kRowB + l16 * 16);
           if (!GATEUP && p.cmb_acc) {
@@ -695,16 +788,21 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
         }
       }
       KNJ_TC_STAMP(tr, 50 + 2 * mat);
-      if (mat + 1 < kEpiMats) asm volatile("bar.sync 5, 384;" ::: "memory");
+      if (mat + 1 < kEpiMats) asm volatile("bar.sync 5, 512;" ::: "memory");
     }
   }
-  if (!ok && p.status) atomicExch(p.status, 1);
+  if (!ok) {
+    // a wait gave up: let the copies that are in flight land before this CTA's shared memory is handed on
+    if (p.status) atomicExch(p.status, 1);
+    const long long t0 = clock64();
+    while (clock64() - t0 < (1ll << 20)) __nanosleep(1000);
+  }
   tc_fence_before();
   __syncthreads();
   // a CTA of a pair may neither free tensor memory nor leave while the peer still reads its accumulators'
   // operands or arrives on its barriers
   if (CG == 2) cluster_sync_all();
-  if (warp == 8) tmem_dealloc<CG>(tmem_base, kTmemCols);
+  if (warp == kMmaWarp) tmem_dealloc<CG>(tmem_base, kTmemCols);
   KNJ_TC_REC(2);
 }
 
@@ -778,12 +876,17 @@ int launch_tc_cg(TcParams p, int max_pairs, cudaStream_t st) {
   }
   if (FMT == 0) {
     const uint64_t rows = (uint64_t)p.n_experts * p.N;
-    int rc = make_row_tensor_map(&p.map0, p.W0, rows, (uint32_t)p.rowBytes, KNJ_Q4K_BYTES, 32);
+    int rc = make_row_tensor_map(&p.map0, p.W0, rows, (uint32_t)p.rowBytes, KNJ_Q4K_BYTES, kRowsM);
     if (rc) return rc;
     if (GATEUP) {
-      rc = make_row_tensor_map(&p.map1, p.W1, rows, (uint32_t)p.rowBytes, KNJ_Q4K_BYTES, 32);
+      rc = make_row_tensor_map(&p.map1, p.W1, rows, (uint32_t)p.rowBytes, KNJ_Q4K_BYTES, kRowsM);
       if (rc) return rc;
     }
+  }
+  {
+    // the rows' number is not known here (a row map may name any row); every index that is read names one that exists
+    const int rc = make_gather_tensor_map(&p.mapx, p.X, 0x7fffffffull, (uint32_t)p.K * 2u);
+    if (rc) return rc;
   }
   // worst case number of token buckets: every expert has a ragged tail
   const long long buckets = (long long)max_pairs / kMaxTok + p.n_experts;

@@ -35,6 +35,9 @@ def ragged_problem(E, F, H, counts, seed):
     (3, 256, 512, [16, 300, 0], 1),   # the same buckets on single SMs (tcgen05 cta_group::1)
     (2, 256, 768, [130, 9], 0),       # 768 = 3 x 256 rows of the down matrix: odd tile count, single-SM form
     (2, 256, 256, [256, 255], 0),     # a full bucket and one token short of it, CTA pairs
+    (4, 256, 1280, [128, 129, 112, 113], 0),  # weights in tensor memory up to 128 tokens, in shared memory above; five superblocks
+    (4, 256, 1280, [128, 129, 15, 17], 1),    # the same on single SMs
+    (3, 768, 256, [128, 384, 65], 0),         # odd tile counts, one matrix: 128 tokens, and a second bucket of 128
 ])
 def test_grouped_gemms(E, F, H, counts, single_sm):
     from kanjoos_b200 import ops, _lib
@@ -84,6 +87,8 @@ def _grouped_gemms(ops, E, F, H, counts):
     (2, 768, 2048, [33, 7], 0),        # the full-size down shape: three superblocks per row
     (2, 512, 384, [130, 9], 0),        # 384 = 3 x 128 rows: odd tile count, single-SM form
     (2, 1024, 256, [256, 255], 1),     # four superblocks per row (the staging's limit), single SMs forced
+    (3, 768, 256, [128, 129, 16], 0),  # weights in tensor memory up to 128 tokens, in shared memory above
+    (2, 512, 384, [128, 1], 0),        # the same on single SMs
 ])
 def test_q6k_down_gemm(E, F, H, counts, single_sm):
     """The grouped down GEMM over Q6_K weights (whole-tile staging, per-slab decode) against the CPU decoder and
@@ -116,4 +121,28 @@ def test_q6k_down_gemm(E, F, H, counts, single_sm):
         if len(rows):
             want[rows] = (a_seen[rows].astype(np.float64) @ Wd[e].astype(np.float64).T).astype(np.float32)
     sty = report(Y.cpu().numpy(), want, f"tc down, Q6_K, E={E} F={F} H={H} counts={counts}")
+    assert sty["unwritten"] == 0 and sty["rel_rmse"] <= TOL
+
+
+@pytest.mark.parametrize("counts", [[130, 9], [128, 0]])
+def test_q4k_down_gemm_one_tile_per_cta(counts):
+    """384 = 3 x 128 output rows: one matrix tile per CTA, a thread unpacks one nibble plane of its row."""
+    from kanjoos_b200 import ops
+    E, F, H, T = 2, 512, 384, sum(counts)
+    rng = np.random.Generator(np.random.Philox([F, H, T]))
+    pe = np.concatenate([np.full(c, e, np.int32) for e, c in enumerate(counts)])
+    pe = pe[rng.permutation(T)]
+    Wd = synth.q4k_rows(rng, E * H, F).reshape(E, H, F // 256, 144)
+    ah = torch.from_numpy((rng.standard_normal((T, F)) * 3.0 / 64.0).astype(np.float16)).cuda()
+    pair_idx, pair_cnt, _, _ = ops.moe_permute(dev(pe), E, T)
+    Y, st = ops.q4k_down_tc(ah, dev(Wd), pair_idx, pair_cnt, T)
+    torch.cuda.synchronize()
+    assert int(st.item()) == 0, "a bounded wait inside the kernel gave up"
+    a_seen = ah.float().cpu().numpy() * 64.0
+    want = np.zeros((T, H), np.float32)
+    for e in range(E):
+        rows = np.nonzero(pe == e)[0]
+        if len(rows):
+            want[rows] = ol.matmul_q4k(Wd[e], np.ascontiguousarray(a_seen[rows]))
+    sty = report(Y.cpu().numpy(), want, f"tc down, one tile, counts={counts}")
     assert sty["unwritten"] == 0 and sty["rel_rmse"] <= TOL
