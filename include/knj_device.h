@@ -29,8 +29,7 @@
  *     allocate and say so where they are declared: knj_moe_stack_create (the
  *     stack launch's scratch), knj_ep_create (the rank's private scratch of the
  *     expert-parallel layer), the residency slot pool and the pinned arena
- *     (knj_residency.h). The library image also carries a 64 KiB device array
- *     per GPU, the scratch of knj_q4k_matmul_noalloc_launch.
+ *     (knj_residency.h).
  *   - Quantized weights are borrowed and immutable: Q4_K superblocks of 144
  *     bytes, row-major [expert][row][K/256][144], base address 16-byte aligned
  *     (KNJ_E_REFUSE otherwise).
@@ -312,14 +311,11 @@ int knj_q4k_matmul_launch(const uint8_t *W, int n_in, int n_out, const void *x, 
  * reference: it exists for callers that may not allocate device memory when
  * they call and have no workspace to lend (a serving loop whose pool is fully
  * committed to resident experts, a plug-in host that only receives input and
- * output buffers, start-up-only allocation policies). Scratch is a fixed array
- * inside the library image, knj_q4k_matmul_noalloc_max_scratch() bytes (64 KiB,
- * enough for 16,256 activation rows),
- * held by every GPU that loads the library until the process exits. Returns
- * KNJ_E_WORKSPACE when knj_q4k_matmul_workspace_bytes(m, n_in) exceeds it. All
- * calls on a device share the array: calls that overlap on the GPU race and must
- * be serialised by the caller. The first call on a device resolves the array's
- * address; make it before any stream capture begins. Calls no allocator. */
+ * output buffers, start-up-only allocation policies). The product needs no
+ * scratch, so calls may overlap. Returns KNJ_E_WORKSPACE when
+ * knj_q4k_matmul_workspace_bytes(m, n_in) exceeds
+ * knj_q4k_matmul_noalloc_max_scratch() (64 KiB: 16,256 activation rows), the
+ * limit of this entry point. Calls no allocator. */
 size_t knj_q4k_matmul_noalloc_max_scratch(void);
 int knj_q4k_matmul_noalloc_launch(const uint8_t *W, int n_in, int n_out, const void *x, int x_dtype, int64_t ldx, int m,
                                   float *y, int64_t ldy, knj_stream_t s);
