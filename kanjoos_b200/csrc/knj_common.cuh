@@ -39,6 +39,9 @@ inline int launch_status(const char *what) {
 inline cudaStream_t as_stream(knj_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 int sm_count();  // SMs of the current device (cached per device)
+// The permutation tables without the active-expert list (knj_router.cu).
+int moe_permute_tables(const int32_t *pair_exp, int P, int E, int idx_stride, int32_t *pair_idx, int32_t *pair_cnt, void *scratch,
+                       size_t scratch_bytes, cudaStream_t st);
 // knj_ep_combine_partial_peer_launch with every owner's array entered at element `parts_off`; with `stage` (f32
 // [T][H], local) the rows of other ranks' tokens are written there instead, one dense block per owner
 int ep_combine_partial_peer_at(const float *Y, const int32_t *pair_exp, const float *pair_w, int T, int H, int k, int exp_lo, int exp_hi,

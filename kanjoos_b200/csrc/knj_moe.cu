@@ -54,7 +54,7 @@ DecodeWs carve_decode(void *base, int T, int H, int F, int E, int k) {
 
 struct PrefillWs {
   float *xn, *logits, *pair_w, *Y;
-  int32_t *pair_exp, *pair_idx, *pair_cnt, *exp_list, *n_active, *status;
+  int32_t *pair_exp, *pair_idx, *pair_cnt, *status;
   void *xh, *ah;
   size_t bytes;
 };
@@ -69,8 +69,6 @@ PrefillWs carve_prefill(void *base, int T, int H, int F, int E, int k) {
   w.pair_w = c.take<float>(P * 4);
   w.pair_idx = c.take<int32_t>((size_t)E * T * 4);
   w.pair_cnt = c.take<int32_t>((size_t)E * 4);
-  w.exp_list = c.take<int32_t>((size_t)E * 4);
-  w.n_active = c.take<int32_t>(16);
   w.status = c.take<int32_t>(16);
   w.xh = c.take<void>((size_t)T * H * 2);
   w.ah = c.take<void>(P * F * 2);
@@ -200,6 +198,8 @@ int knj_moe_ffn_prefill_launch(const knj_moe_ffn_args *a, knj_stream_t s) {
   const PrefillWs w = carve_prefill(a->workspace, T, H, F, E, k);
   const int P = T * k;
 
+  // from here on every launch may be scheduled while its predecessor drains (a chain of dependent launches)
+  KNJ_CUDA(cudaMemsetAsync(w.status, 0, 16, as_stream(s)));  // the GEMMs raise it when a bounded wait gives up
   const void *src = a->x;
   int src_dt = a->x_dtype;
   int64_t src_ld = a->ldx;
@@ -212,7 +212,6 @@ int knj_moe_ffn_prefill_launch(const knj_moe_ffn_args *a, knj_stream_t s) {
   }
   int32_t *pair_exp = a->tap_pair_exp ? a->tap_pair_exp : w.pair_exp;
   float *pair_w = a->tap_pair_w ? a->tap_pair_w : w.pair_w;
-  KNJ_CUDA(cudaMemsetAsync(w.status, 0, 16, as_stream(s)));  // the GEMMs raise it when a bounded wait gives up
   {
     StageSpan sp("moe-router", s);
     rc = knj_router_topk_launch(src, src_dt, src_ld, a->w_router, a->router_bias, T, H, E, k, w.logits, pair_exp, pair_w, s);
@@ -221,8 +220,7 @@ int knj_moe_ffn_prefill_launch(const knj_moe_ffn_args *a, knj_stream_t s) {
   {
     StageSpan sp("moe-gather", s);  // permutation tables and fp16 rows (rows are gathered inside the GEMM)
     // long pair lists take the counting-sort form; its scratch is the activation buffer, which is written later
-    rc = knj_moe_permute_ws_launch(pair_exp, P, E, T, w.pair_idx, w.pair_cnt, w.exp_list, w.n_active, w.ah,
-                                   (size_t)P * F * 2, s);
+    rc = moe_permute_tables(pair_exp, P, E, T, w.pair_idx, w.pair_cnt, w.ah, (size_t)P * F * 2, as_stream(s));
     if (rc) return rc;
     rc = knj_to_f16_launch(src, src_dt, src_ld, T, H, w.xh, s);
     if (rc) return rc;

@@ -312,6 +312,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
   const int warp = warp_index();  // the same register in all lanes: the roles below branch uniformly
   const uint32_t rank = CG == 2 ? cluster_rank() : 0u;  // == blockIdx.x & 1 (m_tiles is even when CG == 2)
 
+  grid_dep_wait();  // the plan and the token rows come from earlier launches
   // ---- which (expert, token bucket) is this CTA's? scan the counts (E <= 256)
   const int m_tile = blockIdx.x % p.m_tiles;
   // every warp finds it for itself: lane l holds the counts of experts 8l..8l+7, a warp scan over the bucket
@@ -808,6 +809,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
 
 // x (f32 / bf16 / f16) -> fp16 with saturation, rows dense
 __global__ void to_f16_kernel(const void *__restrict__ x, int dtype, int64_t ldx, int K, int64_t n, __half *__restrict__ out) {
+  grid_dep_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = i / K, c = i - r * K;
     const float v = load_as_f32(x, dtype, r * ldx + c);
@@ -818,6 +820,7 @@ __global__ void to_f16_kernel(const void *__restrict__ x, int dtype, int64_t ldx
 // the common case, bf16 rows whose length and stride are multiples of 8: 16 bytes in, 16 bytes out per thread and step
 __global__ void __launch_bounds__(256) bf16_to_f16_kernel(const uint4 *__restrict__ x, int64_t ldx8, int K8, int64_t n8,
                                                           uint4 *__restrict__ out) {
+  grid_dep_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = i / K8, c = i - r * K8;
     const uint4 v = __ldg(x + r * ldx8 + c);
@@ -897,13 +900,15 @@ int launch_tc_cg(TcParams p, int max_pairs, cudaStream_t st) {
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = S::kBytes;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = CG;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = g_chain_overlap ? 2 : 1;
   KNJ_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
   return launch_status("q4k_grouped_tc_kernel");
 }
@@ -942,13 +947,13 @@ int knj_to_f16_launch(const void *x, int x_dtype, int64_t ldx, int rows, int K, 
   const int64_t n = (int64_t)rows * K;
   if (x_dtype == KNJ_DT_BF16 && K % 8 == 0 && ldx % 8 == 0 && aligned16(x) && aligned16(out_f16)) {
     const int64_t n8 = n / 8, blocks8 = (n8 + 255) / 256, cap8 = (int64_t)sm_count() * 16;
-    bf16_to_f16_kernel<<<(unsigned)(blocks8 < cap8 ? blocks8 : cap8), 256, 0, as_stream(s)>>>(
-        static_cast<const uint4 *>(x), ldx / 8, K / 8, n8, static_cast<uint4 *>(out_f16));
+    KNJ_CUDA(launch_chain(bf16_to_f16_kernel, dim3((unsigned)(blocks8 < cap8 ? blocks8 : cap8)), dim3(256), 0, as_stream(s),
+                          static_cast<const uint4 *>(x), ldx / 8, K / 8, n8, static_cast<uint4 *>(out_f16)));
     return launch_status("bf16_to_f16_kernel");
   }
   const int64_t blocks = (n + 255) / 256, cap = (int64_t)sm_count() * 16;
-  to_f16_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, as_stream(s)>>>(x, x_dtype, ldx, K, n,
-                                                                                  static_cast<__half *>(out_f16));
+  KNJ_CUDA(launch_chain(to_f16_kernel, dim3((unsigned)(blocks < cap ? blocks : cap)), dim3(256), 0, as_stream(s), x, x_dtype, ldx, K, n,
+                        static_cast<__half *>(out_f16)));
   return launch_status("to_f16_kernel");
 }
 

@@ -18,6 +18,7 @@ namespace {
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const void *__restrict__ x, int dtype, int64_t ldx,
                                                       const __nv_bfloat16 *__restrict__ w, float eps, int H,
                                                       float *__restrict__ out) {
+  grid_dep_wait();
   const int r = blockIdx.x;
   __shared__ float red[8];
   float ss = 0.f;
@@ -163,6 +164,7 @@ __global__ void __launch_bounds__(128) router_logits_mma_kernel(const void *__re
   const int tok0 = blockIdx.y * MT, e0 = blockIdx.x * S::kExperts;
   const int wrow = MT == 64 ? warp * 16 : 0, wexp = MT == 64 ? 0 : warp * 8;  // this warp's part of the tile
   const int nk = H / 32;
+  grid_dep_wait();
 
   auto issue = [&](int kstep, int st) {
     const int k0 = kstep * 32;
@@ -268,6 +270,7 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const float *__restric
                                                           float *__restrict__ pair_w) {
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + (threadIdx.x >> 5);
+  grid_dep_wait();
   if (t >= T) return;
   int sel_e[8];
   float sel_w[8];
@@ -290,6 +293,7 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const float *__restric
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) permute_count_kernel(const int32_t *__restrict__ pair_exp, int P, int E,
                                                             int32_t *__restrict__ counts) {
+  grid_dep_wait();
   __shared__ int hist[256];
   hist[threadIdx.x] = 0;
   __syncthreads();
@@ -304,6 +308,7 @@ __global__ void __launch_bounds__(256) permute_count_kernel(const int32_t *__res
 
 __global__ void __launch_bounds__(256) permute_scan_kernel(int32_t *__restrict__ counts, int chunks, int E, int idx_stride,
                                                            int32_t *__restrict__ pair_cnt) {
+  grid_dep_wait();
   const int e = blockIdx.x;
   __shared__ int wsum[8];
   __shared__ int s_base;
@@ -338,6 +343,7 @@ __global__ void __launch_bounds__(256) permute_scan_kernel(int32_t *__restrict__
 __global__ void __launch_bounds__(256) permute_scatter_kernel(const int32_t *__restrict__ pair_exp, int P, int E,
                                                               const int32_t *__restrict__ base, int idx_stride,
                                                               int32_t *__restrict__ pair_idx) {
+  grid_dep_wait();
   __shared__ int wcnt[8][256];  // per warp and expert: pairs of that expert in the warp, then in the earlier warps
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < 8 * 256; i += 256) (&wcnt[0][0])[i] = 0;
@@ -373,6 +379,7 @@ __global__ void __launch_bounds__(256) permute_scatter_kernel(const int32_t *__r
 __global__ void __launch_bounds__(256) permute_kernel(const int32_t *__restrict__ pair_exp, int P, int idx_stride,
                                                       int32_t *__restrict__ pair_idx,
                                                       int32_t *__restrict__ pair_cnt) {
+  grid_dep_wait();
   const int e = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __shared__ int wsum[8];
@@ -820,7 +827,7 @@ int launch_router_tile(const void *x, int64_t ldx, const __nv_bfloat16 *wr, cons
     }
   }
   const dim3 grid((E + S::kExperts - 1) / S::kExperts, (T + MT - 1) / MT);
-  router_logits_mma_kernel<DT, MT, NSTAGE><<<grid, 128, S::kBytes, st>>>(x, ldx, wr, bias, T, H, E, logits);
+  KNJ_CUDA(launch_chain(router_logits_mma_kernel<DT, MT, NSTAGE>, grid, dim3(128), S::kBytes, st, x, ldx, wr, bias, T, H, E, logits));
   return launch_status("router_logits_mma_kernel");
 }
 // Small tiles while they are at most two CTAs an SM (1184 tokens with 128 experts on 148 SMs); then 64-token tiles, eight
@@ -838,6 +845,29 @@ int launch_router_logits(const void *x, int64_t ldx, const __nv_bfloat16 *wr, co
 
 }  // namespace
 
+namespace knj {
+// pair_idx / pair_cnt alone: what the prefill GEMMs read (the active-expert list is the decode kernels'). Long pair lists
+// with a scratch take the counting sort.
+int moe_permute_tables(const int32_t *pair_exp, int P, int E, int idx_stride, int32_t *pair_idx, int32_t *pair_cnt, void *scratch,
+                       size_t scratch_bytes, cudaStream_t st) {
+  if (P < 8192 || !scratch) {
+    KNJ_CUDA(launch_chain(permute_kernel, dim3(E), dim3(256), 0, st, pair_exp, P, idx_stride, pair_idx, pair_cnt));
+    return launch_status("permute_kernel");
+  }
+  if (scratch_bytes < knj_moe_permute_scratch_bytes(P, E)) {
+    set_error("knj_moe_permute_ws: scratch of %zu bytes needed, %zu given", knj_moe_permute_scratch_bytes(P, E), scratch_bytes);
+    return KNJ_E_WORKSPACE;
+  }
+  const int chunks = (P + 255) / 256;
+  int32_t *counts = static_cast<int32_t *>(scratch);
+  KNJ_CUDA(cudaMemsetAsync(pair_idx, 0xff, (size_t)E * idx_stride * sizeof(int32_t), st));  // -1 padding
+  KNJ_CUDA(launch_chain(permute_count_kernel, dim3(chunks), dim3(256), 0, st, pair_exp, P, E, counts));
+  KNJ_CUDA(launch_chain(permute_scan_kernel, dim3(E), dim3(256), 0, st, counts, chunks, E, idx_stride, pair_cnt));
+  KNJ_CUDA(launch_chain(permute_scatter_kernel, dim3(chunks), dim3(256), 0, st, pair_exp, P, E, counts, idx_stride, pair_idx));
+  return launch_status("permute_scatter_kernel");
+}
+}  // namespace knj
+
 extern "C" {
 
 int knj_rmsnorm_launch(const void *x, int x_dtype, int64_t ldx, const uint16_t *w_bf16, float eps, int T, int H,
@@ -845,8 +875,8 @@ int knj_rmsnorm_launch(const void *x, int x_dtype, int64_t ldx, const uint16_t *
   KNJ_REQUIRE(x && w_bf16 && out, "knj_rmsnorm: null pointer");
   KNJ_REQUIRE(H > 0 && x_dtype >= KNJ_DT_F32 && x_dtype <= KNJ_DT_F16, "knj_rmsnorm: bad H / dtype");
   if (T <= 0) return KNJ_OK;
-  rmsnorm_kernel<<<T, 256, 0, as_stream(s)>>>(x, x_dtype, ldx, reinterpret_cast<const __nv_bfloat16 *>(w_bf16), eps, H,
-                                              out);
+  KNJ_CUDA(launch_chain(rmsnorm_kernel, dim3(T), dim3(256), 0, as_stream(s), x, x_dtype, ldx, reinterpret_cast<const __nv_bfloat16 *>(w_bf16), eps, H,
+                                              out));
   return launch_status("rmsnorm_kernel");
 }
 
@@ -871,7 +901,7 @@ int knj_router_topk_launch(const void *x, int x_dtype, int64_t ldx, const uint16
     rc = launch_status("router_logits_kernel");
   }
   if (rc) return rc;
-  router_topk_kernel<<<(T + 3) / 4, 128, 0, as_stream(s)>>>(logits, T, E, k, pair_exp, pair_w);
+  KNJ_CUDA(launch_chain(router_topk_kernel, dim3((T + 3) / 4), dim3(128), 0, as_stream(s), logits, T, E, k, pair_exp, pair_w));
   return launch_status("router_topk_kernel");
 }
 
@@ -886,25 +916,9 @@ int knj_moe_permute_ws_launch(const int32_t *pair_exp, int P, int E, int idx_str
                               int32_t *exp_list, int32_t *n_active, void *scratch, size_t scratch_bytes, knj_stream_t s) {
   KNJ_REQUIRE(pair_exp && pair_idx && pair_cnt && exp_list && n_active, "knj_moe_permute_ws: null pointer");
   KNJ_REQUIRE(P >= 0 && E >= 1 && E <= 256 && idx_stride >= 1, "knj_moe_permute_ws: bad sizes (E <= 256)");
-  if (P < 8192 || !scratch) return knj_moe_permute_launch(pair_exp, P, E, idx_stride, pair_idx, pair_cnt, exp_list, n_active, s);
-  if (scratch_bytes < knj_moe_permute_scratch_bytes(P, E)) {
-    set_error("knj_moe_permute_ws: scratch of %zu bytes needed, %zu given", knj_moe_permute_scratch_bytes(P, E), scratch_bytes);
-    return KNJ_E_WORKSPACE;
-  }
-  cudaStream_t st = as_stream(s);
-  const int chunks = (P + 255) / 256;
-  int32_t *counts = static_cast<int32_t *>(scratch);
-  KNJ_CUDA(cudaMemsetAsync(pair_idx, 0xff, (size_t)E * idx_stride * sizeof(int32_t), st));  // -1 padding
-  permute_count_kernel<<<chunks, 256, 0, st>>>(pair_exp, P, E, counts);
-  int rc = launch_status("permute_count_kernel");
+  const int rc = moe_permute_tables(pair_exp, P, E, idx_stride, pair_idx, pair_cnt, scratch, scratch_bytes, as_stream(s));
   if (rc) return rc;
-  permute_scan_kernel<<<E, 256, 0, st>>>(counts, chunks, E, idx_stride, pair_cnt);
-  rc = launch_status("permute_scan_kernel");
-  if (rc) return rc;
-  permute_scatter_kernel<<<chunks, 256, 0, st>>>(pair_exp, P, E, counts, idx_stride, pair_idx);
-  rc = launch_status("permute_scatter_kernel");
-  if (rc) return rc;
-  active_list_kernel<<<1, 256, 0, st>>>(pair_cnt, E, exp_list, n_active);
+  active_list_kernel<<<1, 256, 0, as_stream(s)>>>(pair_cnt, E, exp_list, n_active);
   return launch_status("active_list_kernel");
 }
 
@@ -912,8 +926,7 @@ int knj_moe_permute_launch(const int32_t *pair_exp, int P, int E, int idx_stride
                            int32_t *exp_list, int32_t *n_active, knj_stream_t s) {
   KNJ_REQUIRE(pair_exp && pair_idx && pair_cnt && exp_list && n_active, "knj_moe_permute: null pointer");
   KNJ_REQUIRE(P >= 0 && E >= 1 && idx_stride >= 1, "knj_moe_permute: bad sizes");
-  permute_kernel<<<E, 256, 0, as_stream(s)>>>(pair_exp, P, idx_stride, pair_idx, pair_cnt);
-  int rc = launch_status("permute_kernel");
+  const int rc = moe_permute_tables(pair_exp, P, E, idx_stride, pair_idx, pair_cnt, nullptr, 0, as_stream(s));
   if (rc) return rc;
   active_list_kernel<<<1, 256, 0, as_stream(s)>>>(pair_cnt, E, exp_list, n_active);
   return launch_status("active_list_kernel");
