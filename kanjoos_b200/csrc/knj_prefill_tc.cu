@@ -72,6 +72,7 @@ struct TcParams {
   int64_t idxStride;
   float out_scale;
   int *status;
+  int chained;             // launched with programmatic serialization
   // fused weighted combine (single-matrix form only; cmb_acc == null: off): instead of storing the per-pair row,
   // the epilogue adds cmb_w[pair] * row into cmb_acc[pair / cmb_div] with vector reductions in L2
   const float *cmb_w;
@@ -312,7 +313,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
   const int warp = warp_index();  // the same register in all lanes: the roles below branch uniformly
   const uint32_t rank = CG == 2 ? cluster_rank() : 0u;  // == blockIdx.x & 1 (m_tiles is even when CG == 2)
 
-  grid_dep_wait();  // the plan and the token rows come from earlier launches
+  if (p.chained) grid_dep_wait();  // the plan and the token rows come from earlier launches
   // ---- which (expert, token bucket) is this CTA's? scan the counts (E <= 256)
   const int m_tile = blockIdx.x % p.m_tiles;
   // every warp finds it for itself: lane l holds the counts of experts 8l..8l+7, a warp scan over the bucket
@@ -894,6 +895,10 @@ int launch_tc_cg(TcParams p, int max_pairs, cudaStream_t st) {
   // worst case number of token buckets: every expert has a ragged tail
   const long long buckets = (long long)max_pairs / kMaxTok + p.n_experts;
   const long long grid = buckets * p.m_tiles;
+  // Overlapping the launch with its predecessor's end saves a few microseconds and costs every CTA a wait: only grids of up
+  // to sixteen waves (with every grid chained a step of 16384 tokens took 1886 us and 4001 Q6_K ones 677, with the rule
+  // 1833 and 666; at 100 tokens the chain is worth 242 -> 228).
+  p.chained = g_chain_overlap && grid <= 16ll * sm_count();
   KNJ_REQUIRE(grid > 0 && grid < (1ll << 31), "grouped GEMM: grid of %lld CTAs out of range", grid);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid);
@@ -908,7 +913,7 @@ int launch_tc_cg(TcParams p, int max_pairs, cudaStream_t st) {
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = g_chain_overlap ? 2 : 1;
+  cfg.numAttrs = p.chained ? 2 : 1;
   KNJ_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
   return launch_status("q4k_grouped_tc_kernel");
 }
