@@ -302,10 +302,15 @@ int knj_fuse_gateup_silu_launch(const float *G, const float *U, void *A, int a_d
 
 /* Single-matrix GEMV/GEMM convenience (the CPU path's Model::matmul,
  * src/model/model.cpp:326-380): y[m][n_out] = x[m][n_in] . W^T, W Q4_K
- * [n_out][n_in/256][144]. workspace >= knj_q4k_matmul_workspace_bytes(m, n_in). */
+ * [n_out][n_in/256][144]. workspace >= knj_q4k_matmul_workspace_bytes(m, n_in).
+ * There is no status word: if a bounded wait of the kernel gives up
+ * (knj_decode_wait_limit), the outputs of the work units it concerns are NaN. */
 size_t knj_q4k_matmul_workspace_bytes(int m, int n_in);
 int knj_q4k_matmul_launch(const uint8_t *W, int n_in, int n_out, const void *x, int x_dtype, int64_t ldx, int m,
                           float *y, int64_t ldy, void *workspace, size_t workspace_bytes, knj_stream_t s);
+/* Test hook of the calling thread: 1 = in its next products one wait of the first
+ * thread block cannot be met and runs into its limit; 0 = off (default). */
+void knj_q4k_matmul_test_stall(int on);
 
 /* Allocation-free form of knj_q4k_matmul_launch. No counterpart in the
  * reference: it exists for callers that may not allocate device memory when

@@ -171,6 +171,7 @@ SIGNATURES = {
     "knj_moe_acc_finish_launch": (_i, [_vp, _vp, _i, _i64, _i, _i, _vp]),
     "knj_fuse_gateup_silu_launch": (_i, [_vp, _vp, _vp, _i, _i64, _vp]),
     "knj_q4k_matmul_workspace_bytes": (_sz, [_i, _i]),
+    "knj_q4k_matmul_test_stall": (None, [_i]),
     "knj_q4k_matmul_launch": (_i, [_vp, _i, _i, _vp, _i, _i64, _i, _vp, _i64, _vp, _sz, _vp]),
     "knj_q4k_matmul_noalloc_max_scratch": (_sz, []),
     "knj_q4k_matmul_noalloc_launch": (_i, [_vp, _i, _i, _vp, _i, _i64, _i, _vp, _i64, _vp]),

@@ -44,6 +44,7 @@ struct ProjParams {
   int64_t idxStride;
   int *status;    // optional: set to 1 when a bounded wait gave up
   long long wait_cycles;   // limit of every wait inside the kernel
+  int stall;      // test hook: the first box of CTA 0's first warp never counts as landed
   CUtensorMap map0, map1;  // TMA descriptors of W0 / W1: box = sbs superblocks x 8 (dual) or 16 rows
 };
 
@@ -85,7 +86,8 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_proj_kernel(const __grid_cons
   sm.pair = s_pair;
   sm.fail = &s_fail;
   if (lane == 0)
-    for (int s = 0; s < q4e::kMaxStages; ++s) mbar_init(&sm.bars[warp * q4e::kMaxStages + s], 1);
+    for (int s = 0; s < q4e::kMaxStages; ++s)
+      mbar_init(&sm.bars[warp * q4e::kMaxStages + s], p.stall && blockIdx.x == 0 && warp == 0 && s == 0 ? 2 : 1);
   if (threadIdx.x == 0) s_fail = 0;
   mbar_init_fence();
   grid_dep_wait();  // the plan and the activation rows come from earlier launches
@@ -127,9 +129,23 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_proj_kernel(const __grid_cons
       [&](int row, int sb, int ln, float (&v)[8]) { q4e::load8_f32(p.X, p.x_dtype, (int64_t)row * p.ldx + 256 * sb + 8 * ln, v); },
       tmode);
   if (!ok && lane == 0 && p.status) atomicExch(p.status, 1);
+  if (IDENT) {
+    // A dense product has no status word: where a wait gave up, all outputs of this CTA's units become NaN, so that a
+    // caller cannot take what the buffer held before for a result.
+    __syncthreads();
+    if (*sm.fail) {
+      const int tiles = p.shape.tiles;
+      for (long long i = threadIdx.x; i < (long long)(u1 - u0) * q4e::kJobTok * 16; i += kThreads) {
+        const int u = u0 + (int)(i / (q4e::kJobTok * 16)), tk = (int)(i / 16) % q4e::kJobTok;
+        const int tok = u / tiles * q4e::kJobTok + tk;
+        if (tok < p.n_ident) p.out0[(size_t)tok * p.shape.N + u % tiles * 16 + (int)(i % 16)] = __int_as_float(0x7fffffff);
+      }
+    }
+  }
 }
 
 long long g_decode_wait_cycles = kMaxWaitCycles;
+thread_local int t_stall_dense = 0;  // knj_q4k_matmul_test_stall
 
 template <bool DUAL, bool IDENT = false>
 int launch_proj(ProjParams p, int n_experts_max, cudaStream_t st) {
@@ -195,7 +211,7 @@ int dense_product(const uint8_t *W, int n_in, int n_out, const void *x, int x_dt
   ProjParams p{};
   p.W0 = W; p.X = x; p.x_dtype = x_dtype; p.ldx = ldx; p.n_ident = m;
   p.out0 = y; p.shape.N = n_out; p.K = n_in; p.row_div = 1;
-  p.shape.tiles = n_out / 16; p.idxStride = m;
+  p.shape.tiles = n_out / 16; p.idxStride = m; p.stall = t_stall_dense;
   return launch_proj<false, true>(p, 1, as_stream(s));
 }
 
@@ -259,6 +275,8 @@ int knj_q4k_proj_launch(const void *A, int a_dtype, int64_t lda, const uint8_t *
   p.shape.tiles = N / 16; p.idxStride = idxStride; p.status = status;
   return launch_proj<false>(p, n_experts, as_stream(s));
 }
+
+void knj_q4k_matmul_test_stall(int on) { t_stall_dense = on & 1; }
 
 size_t knj_q4k_matmul_workspace_bytes(int m, int n_in) {
   if (m <= 0 || n_in <= 0) return 0;

@@ -195,7 +195,7 @@ def q4k_matmul(W: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
     n_out, nsb, _ = W.shape
     m, n_in = x.shape
     assert nsb * 256 == n_in
-    y = torch.empty((m, n_out), dtype=torch.float32, device="cuda")  # every element is written
+    y = torch.empty((m, n_out), dtype=torch.float32, device="cuda")  # every element is written (NaN where a bounded wait gave up)
     nbytes = lib().knj_q4k_matmul_workspace_bytes(m, n_in)
     ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
     check(lib().knj_q4k_matmul_launch(_p(W), n_in, n_out, _p(x), _DT[x.dtype], n_in, m, _p(y), n_out, _p(ws), nbytes,

@@ -15,6 +15,20 @@ pytestmark = pytest.mark.gpu
 TOL_F32 = 1e-5
 
 
+def product_into(W, x, y):
+    """knj_q4k_matmul_launch into the caller's y (which the tests poison first)."""
+    import ctypes as C
+    from kanjoos_b200 import _lib, ops
+    L = _lib.lib()
+    (m, n_in), n_out = x.shape, W.shape[0]
+    nbytes = L.knj_q4k_matmul_workspace_bytes(m, n_in)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    _lib.check(L.knj_q4k_matmul_launch(C.c_void_p(W.data_ptr()), n_in, n_out, C.c_void_p(x.data_ptr()), ops._DT[x.dtype],
+                                       n_in, m, C.c_void_p(y.data_ptr()), n_out, C.c_void_p(ws.data_ptr()), nbytes,
+                                       C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    return y
+
+
 def test_dequant_crafted_blocks_bit_exact(golden):
     from kanjoos_b200 import ops
     got = ops.q4k_dequant(dev(golden["q4k_blocks"])).cpu().numpy()
@@ -107,6 +121,37 @@ def test_matmul_wide_dynamic_range():
             assert np.all(got[r] == 0.0)
             continue
         assert report(got[r], want[r], f"row {r}")["rel_rmse"] <= 2e-5
+
+
+@pytest.mark.parametrize("m,n_out,nan_rows", [
+    (5, 4096, 4),   # two jobs of 256 tiles over the SMs: the first block holds the first tiles of rows 0..3
+    (1, 4096, 1),   # one job, K split over the warps of a tile
+])
+def test_a_wait_that_gives_up_leaves_nan(m, n_out, nan_rows):
+    """The product has no status word: where a bounded wait runs out the outputs must be NaN, not what the buffer
+    held before, and everything the other blocks computed stays right. The hook withholds one arrival, the copy
+    itself lands."""
+    from kanjoos_b200 import _lib, ops
+    L = _lib.lib()
+    rng = np.random.Generator(np.random.Philox([m, n_out]))
+    W = dev(synth.q4k_rows(rng, n_out, 1024))
+    x = dev(rng.standard_normal((m, 1024)).astype(np.float32))
+    want = ops.q4k_matmul(W, x)
+    y = torch.full((m, n_out), SENTINEL, dtype=torch.float32, device="cuda")
+    L.knj_decode_wait_limit(2_000_000)  # about a millisecond
+    L.knj_q4k_matmul_test_stall(1)
+    try:
+        product_into(W, x, y)
+        torch.cuda.synchronize()
+    finally:
+        L.knj_q4k_matmul_test_stall(0)
+        L.knj_decode_wait_limit(0)
+    bad = torch.isnan(y)
+    assert bad[:nan_rows, :16].all(), "outputs of a given-up tile must be NaN"
+    assert not (y == SENTINEL).any() and int(bad.sum()) < y.numel() // 16
+    assert torch.equal(y[~bad], want[~bad])
+    product_into(W, x, y)  # the context and the kernel stay usable
+    assert torch.equal(y, want)
 
 
 def test_refusals_do_not_launch():
