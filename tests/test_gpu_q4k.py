@@ -68,7 +68,9 @@ def test_cfg1_gemv(golden):
     from kanjoos_b200 import ops
     W = synth.q4k_rows(synth.stream(1, "gate"), synth.FFN, synth.HIDDEN)
     x = synth.stream(1, "x").standard_normal(synth.HIDDEN).astype(np.float32)
-    got = ops.q4k_matmul(dev(W), dev(x[None])).cpu().numpy()[0]
+    y = torch.full((1, synth.FFN), SENTINEL, dtype=torch.float32, device="cuda")
+    got = product_into(dev(W), dev(x[None]), y).cpu().numpy()[0]
+    assert np.array_equal(ops.q4k_matmul(dev(W), dev(x[None])).cpu().numpy()[0], got)
     st = report(got, golden["cfg1_y"], "cfg1 GEMV vs reference dequant_dot_f32")
     assert st["unwritten"] == 0 and st["rel_rmse"] <= TOL_F32
     # and against an exact (float64) product of the bit-exact decode
@@ -80,11 +82,10 @@ def test_cfg1_gemv(golden):
 @pytest.mark.parametrize("m", [1, 2, 4, 5, 15, 16, 17, 64])
 @pytest.mark.parametrize("n_in,n_out", [(256, 16), (768, 48), (2048, 64)])
 def test_matmul_ragged_row_counts(m, n_in, n_out):
-    from kanjoos_b200 import ops
     rng = np.random.Generator(np.random.Philox([m, n_in, n_out]))
     W = synth.q4k_rows(rng, n_out, n_in)
     x = rng.standard_normal((m, n_in)).astype(np.float32)
-    got = ops.q4k_matmul(dev(W), dev(x)).cpu().numpy()
+    got = product_into(dev(W), dev(x), torch.full((m, n_out), SENTINEL, dtype=torch.float32, device="cuda")).cpu().numpy()
     want = ol.matmul_q4k(W, x)
     st = report(got, want, f"matmul m={m} {n_out}x{n_in}")
     assert st["unwritten"] == 0 and st["rel_rmse"] <= TOL_F32
