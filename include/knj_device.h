@@ -319,8 +319,8 @@ void knj_q4k_matmul_test_stall(int on);
  * output buffers, start-up-only allocation policies). The product needs no
  * scratch, so calls may overlap. Returns KNJ_E_WORKSPACE when
  * knj_q4k_matmul_workspace_bytes(m, n_in) exceeds
- * knj_q4k_matmul_noalloc_max_scratch() (64 KiB: 16,256 activation rows), the
- * limit of this entry point. Calls no allocator. */
+ * knj_q4k_matmul_noalloc_max_scratch() (64 KiB: 16,320 activation rows): a limit
+ * of this entry point only, no memory of that size exists. Calls no allocator. */
 size_t knj_q4k_matmul_noalloc_max_scratch(void);
 int knj_q4k_matmul_noalloc_launch(const uint8_t *W, int n_in, int n_out, const void *x, int x_dtype, int64_t ldx, int m,
                                   float *y, int64_t ldy, knj_stream_t s);

@@ -307,12 +307,13 @@ int knj_q4k_matmul_launch(const uint8_t *W, int n_in, int n_out, const void *x, 
 // buffers, and callers that forbid allocator calls after start-up because an
 // allocation can synchronise the device or fragment a tightly packed HBM budget.
 //
-// The product needs no scratch: the one-matrix plan is derived in the kernel.
-// Problems whose workspace would exceed kNoAllocScratchBytes are refused with
-// KNJ_E_WORKSPACE, the limit this entry point has always had. Calls may overlap.
+// The product needs no scratch (the one-matrix plan is derived in the kernel),
+// so calls may overlap. Problems whose workspace would exceed
+// kNoAllocScratchBytes are refused with KNJ_E_WORKSPACE: a limit of this entry
+// point and nothing more, kept so that what it refused it goes on refusing.
 // ---------------------------------------------------------------------------
 namespace {
-constexpr size_t kNoAllocScratchBytes = (size_t)64 << 10;  // the pair list of up to 16,256 activation rows
+constexpr size_t kNoAllocScratchBytes = (size_t)64 << 10;  // the workspace of 16,320 activation rows
 }  // namespace
 
 size_t knj_q4k_matmul_noalloc_max_scratch(void) { return kNoAllocScratchBytes; }
@@ -322,7 +323,7 @@ int knj_q4k_matmul_noalloc_launch(const uint8_t *W, int n_in, int n_out, const v
   KNJ_REQUIRE(m > 0 && n_in > 0, "knj_q4k_matmul_noalloc: m and n_in must be positive");
   const size_t need = knj_q4k_matmul_workspace_bytes(m, n_in);
   if (need > kNoAllocScratchBytes) {
-    set_error("knj_q4k_matmul_noalloc: m=%d rows of n_in=%d need %zu bytes of scratch, the built-in array holds %zu; "
+    set_error("knj_q4k_matmul_noalloc: m=%d rows of n_in=%d (a workspace of %zu bytes) are above this entry point's limit of %zu; "
               "use knj_q4k_matmul_launch with a caller workspace",
               m, n_in, need, kNoAllocScratchBytes);
     return KNJ_E_WORKSPACE;

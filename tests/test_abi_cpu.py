@@ -96,6 +96,17 @@ CAPS = dict(Dot4I32I8=0, Dot8I32I4=1, PkFmaF16=2, WmmaF16=3, Fp8=4, Sdot4Builtin
             TmaBulk=9)
 
 
+def test_noalloc_product_limit(L):
+    """The row limit of the allocation-free product, decided on the host before anything touches a device."""
+    limit = L.knj_q4k_matmul_noalloc_max_scratch()
+    assert limit == 64 << 10
+    assert L.knj_q4k_matmul_workspace_bytes(16320, 256) <= limit < L.knj_q4k_matmul_workspace_bytes(16321, 256)
+    some = C.c_void_p(4096)  # never read: the call is refused first
+    assert L.knj_q4k_matmul_noalloc_launch(some, 256, 16, some, 0, 256, 16321, some, 16, None) == -4
+    msg = L.knj_last_error_string().decode()
+    assert "16321 rows" in msg and "limit of 65536" in msg and "knj_q4k_matmul_launch" in msg
+
+
 def test_check_arch_verdicts(L):
     reason = C.c_char_p()
     assert L.knj_check_arch_c(None, b"sm_100", C.byref(reason)) == 1 and b"KNJ_BUILD_ARCH is not set" in reason.value
