@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_proj_kernel(const __grid_cons
   sm.fail = &s_fail;
   if (lane == 0)
     for (int s = 0; s < q4e::kMaxStages; ++s)
-      mbar_init(&sm.bars[warp * q4e::kMaxStages + s], p.stall && blockIdx.x == 0 && warp == 0 && s == 0 ? 2 : 1);
+      mbar_init(&sm.bars[warp * q4e::kMaxStages + s], IDENT && p.stall && blockIdx.x == 0 && warp == 0 && s == 0 ? 2 : 1);
   if (threadIdx.x == 0) s_fail = 0;
   mbar_init_fence();
   grid_dep_wait();  // the plan and the activation rows come from earlier launches
