@@ -299,3 +299,52 @@ def test_prefill_combine_forms_with_residual_and_bf16_output(cfg2):
     assert np.mean(fused != o1) < 0.01 and report(fused, o1, "fused vs ordered, bf16 out + residual")["rel_rmse"] <= 5e-3
     want, _, _ = ol.moe(wr, bank, hx)
     assert report(o1, synth.bf16_round(hx + want), "ordered, residual, bf16 out vs CPU path")["rel_rmse"] <= 5e-3
+
+
+@pytest.mark.parametrize("T,down,norm", [
+    (20, "q4k", True),     # fewer than 32 tokens: the plain router launch inside the chain
+    (100, "q4k", False),
+    (600, "q6k", True),
+    (1200, "q4k", True),   # 9600 pairs: the counting sort, which starts with a memset
+    (3000, "q6k", False),
+])
+def test_launch_chain_off_on_and_captured(T, down, norm):
+    """The layer launches form chains of dependent launches. Alone (overlap off), chained back to back over changing
+    inputs with one workspace, and replayed from a captured graph they must give the same bits: a kernel that read a
+    predecessor's output too early would not."""
+    from kanjoos_b200 import _lib
+    E, H, F, k = 16, 512, 256, 8
+    bank = synth.expert_bank(106, n_experts=E, hidden=H, ffn=F)
+    wr, _ = synth.router_weight(106, n_experts=E, hidden=H)
+    if down == "q6k":
+        rng = np.random.Generator(np.random.Philox(106))
+        W6 = rng.integers(0, 256, size=(E, H, F // 256, 210), dtype=np.uint8)
+        W6[..., 208:210] = (np.abs(rng.standard_normal((E, H, F // 256, 1))) * 0.01).astype(np.float16).view(np.uint8)
+        bank = dict(bank, down=W6)
+    layer = make_layer(bank, wr, k, T, norm=synth.norm_weight(106, 0, H) if norm else None, residual=norm)
+    xs = [dev(synth.hidden_rows(106, T, H, layer=l)).to(torch.bfloat16) for l in range(5)]
+    for fn in (layer.prefill, layer.decode):
+        outs = [[torch.full((T, H), float("nan"), device="cuda") for _ in xs] for _ in range(4)]
+        L = _lib.lib()
+        try:
+            L.knj_launch_overlap(0)
+            for x, o in zip(xs, outs[0]):
+                fn(x, out=o)
+                torch.cuda.synchronize()
+        finally:
+            L.knj_launch_overlap(1)
+        for r in (1, 2, 3):
+            for x, o in zip(xs, outs[r]):
+                fn(x, out=o)
+        torch.cuda.synchronize()
+        for r in (1, 2, 3):
+            for o, want in zip(outs[r], outs[0]):
+                assert not torch.isnan(want).any() and torch.equal(o, want)
+        xin, out = xs[0].clone(), torch.empty((T, H), device="cuda")
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            fn(xin, out=out)
+        for x, want in zip(xs[1:], outs[0][1:]):
+            xin.copy_(x)
+            g.replay()
+            assert torch.equal(out, want)
