@@ -338,10 +338,11 @@ int knj_to_f16_launch(const void *x, int x_dtype, int64_t ldx, int rows, int K, 
  * 0 (default) = CTA pairs wherever the tile count is even. Process-wide. */
 void knj_q4k_tc_single_sm(int on);
 
-/* Launch mode of the kernels of a decode layer (no reference counterpart).
- * 1 (default): programmatic stream serialization -- each grid may be scheduled
- * while its predecessor on the stream drains and waits on the device for the
- * predecessor's completion before reading its results; 0: plain launches. */
+/* Launch mode of the kernels of the layer launches, decode and prefill, and of
+ * the dense product (no reference counterpart). 1 (default): programmatic stream
+ * serialization -- a grid may be scheduled before its predecessor on the stream
+ * has completed and waits on the device for that before it reads anything;
+ * 0: plain launches. Process-wide; the results are the same. */
 void knj_launch_overlap(int on);
 
 /* Grouped gate+up GEMM over per-expert token buckets on the tensor cores

@@ -53,9 +53,10 @@ int ep_combine_partial_peer_f16_at(const float *Y, const int32_t *pair_exp, cons
 int ep_reduce_sel_f16(const float *parts, int n_ranks, int T_loc, int H, const int32_t *pair_exp, int k, int experts_per_rank,
                       const void *resid, int resid_dtype, void *out, int out_dtype, cudaStream_t s);
 
-// Launch of a kernel that belongs to a chain of dependent launches on one stream (the decode layer). With
+// Launch of a kernel that belongs to a chain of dependent launches on one stream (the layer launches). With
 // overlap on, the launch carries the programmatic-stream-serialization attribute: the grid may be scheduled
-// while its predecessor drains, and it must call grid_dep_wait() before it touches anything the predecessor
+// before its predecessor has completed (from grid_dep_signal() on where the predecessor calls it, else as the
+// predecessor's blocks exit), and it must call grid_dep_wait() before it touches anything the predecessor
 // wrote. Off (knj_launch_overlap(0)): a plain launch; grid_dep_wait() is then a no-op.
 extern int g_chain_overlap;
 template <class... KArgs, class... Args>
@@ -98,12 +99,15 @@ void small_stack_destroy(SmallStack *st);
 // ---- device helpers --------------------------------------------------------
 #if defined(__CUDACC__)
 
-// Blocks until the grids this launch depends on have completed and their writes are visible; then lets the
-// next launch of the chain be scheduled early. No-ops for a plain launch.
-__device__ __forceinline__ void grid_dep_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
+// Blocks until the grids this launch depends on have completed and their writes are visible. A no-op for a plain launch.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next launch of the chain take its places while this grid still runs (once every block has called this or
+// exited). Only the decode layer's front and projection kernels do, grids of one block per SM or less. After a larger
+// grid the next one's blocks take what places are left and run worse from there than launched at its end: signalled by
+// the row normalisation, the router made a layer of 512 tokens 284 us long, not signalled 247; signalled by the down
+// GEMM, the combine cost 4 us at 100 tokens and 45 at 16384 (hidden 2048, 128 experts; hidden 1024, 32 experts at 16384
+// tokens 822 -> 760 us).
+__device__ __forceinline__ void grid_dep_signal() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));

@@ -198,7 +198,8 @@ int knj_moe_ffn_prefill_launch(const knj_moe_ffn_args *a, knj_stream_t s) {
   const PrefillWs w = carve_prefill(a->workspace, T, H, F, E, k);
   const int P = T * k;
 
-  // from here on every launch may be scheduled while its predecessor drains (a chain of dependent launches)
+  // A chain of dependent launches: each but the router's for fewer than 32 tokens and the two of the fused combine's
+  // accumulator is prepared while its predecessor ends; what follows a memset (this one, the counting sort's) starts anew.
   KNJ_CUDA(cudaMemsetAsync(w.status, 0, 16, as_stream(s)));  // the GEMMs raise it when a bounded wait gives up
   const void *src = a->x;
   int src_dt = a->x_dtype;

@@ -72,7 +72,6 @@ struct TcParams {
   int64_t idxStride;
   float out_scale;
   int *status;
-  int chained;             // launched with programmatic serialization
   // fused weighted combine (single-matrix form only; cmb_acc == null: off): instead of storing the per-pair row,
   // the epilogue adds cmb_w[pair] * row into cmb_acc[pair / cmb_div] with vector reductions in L2
   const float *cmb_w;
@@ -313,7 +312,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
   const int warp = warp_index();  // the same register in all lanes: the roles below branch uniformly
   const uint32_t rank = CG == 2 ? cluster_rank() : 0u;  // == blockIdx.x & 1 (m_tiles is even when CG == 2)
 
-  if (p.chained) grid_dep_wait();  // the plan and the token rows come from earlier launches
+  grid_dep_wait();  // the plan and the token rows come from earlier launches
   // ---- which (expert, token bucket) is this CTA's? scan the counts (E <= 256)
   const int m_tile = blockIdx.x % p.m_tiles;
   // every warp finds it for itself: lane l holds the counts of experts 8l..8l+7, a warp scan over the bucket
@@ -895,10 +894,6 @@ int launch_tc_cg(TcParams p, int max_pairs, cudaStream_t st) {
   // worst case number of token buckets: every expert has a ragged tail
   const long long buckets = (long long)max_pairs / kMaxTok + p.n_experts;
   const long long grid = buckets * p.m_tiles;
-  // Overlapping the launch with its predecessor's end saves a few microseconds and costs every CTA a wait: only grids of up
-  // to sixteen waves (with every grid chained a step of 16384 tokens took 1886 us and 4001 Q6_K ones 677, with the rule
-  // 1833 and 666; at 100 tokens the chain is worth 242 -> 228).
-  p.chained = g_chain_overlap && grid <= 16ll * sm_count();
   KNJ_REQUIRE(grid > 0 && grid < (1ll << 31), "grouped GEMM: grid of %lld CTAs out of range", grid);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid);
@@ -910,10 +905,12 @@ int launch_tc_cg(TcParams p, int max_pairs, cudaStream_t st) {
   attr[0].val.clusterDim.x = CG;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  // Part of the chain at every size: its launch is prepared while the predecessor ends. 100 tokens 215.4 -> 210.5 us against
+  // plain launches, 1000 261 -> 257, 4001 499 -> 494, 16384 1747 -> 1742 (both GEMMs of a layer, neither signals early).
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = p.chained ? 2 : 1;
+  cfg.numAttrs = g_chain_overlap ? 2 : 1;
   KNJ_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
   return launch_status("q4k_grouped_tc_kernel");
 }

@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_proj_kernel(const __grid_cons
   if (threadIdx.x == 0) s_fail = 0;
   mbar_init_fence();
   grid_dep_wait();  // the plan and the activation rows come from earlier launches
+  grid_dep_signal();
 
   // ---- the job table: jobs per active expert, exclusive prefix (every CTA derives the same table)
   const int n_act = IDENT ? 1 : min(p.n_active[0], 256);

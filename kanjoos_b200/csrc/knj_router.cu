@@ -670,6 +670,7 @@ __global__ void __launch_bounds__(256) moe_front_kernel(const FrontParams p) {
     // the router and norm weights above do not depend on the previous launch and are already on their way;
     // the token rows are the previous layer's output
     grid_dep_wait();
+    grid_dep_signal();
     KNJ_FRONT_STAMP(6);
     if (nt > 0) fetch(t0, ra);
     for (int i = 0; i < nt; i += 2) {
