@@ -58,6 +58,10 @@ int ep_reduce_sel_f16(const float *parts, int n_ranks, int T_loc, int H, const i
 // before its predecessor has completed (from grid_dep_signal() on where the predecessor calls it, else as the
 // predecessor's blocks exit), and it must call grid_dep_wait() before it touches anything the predecessor
 // wrote. Off (knj_launch_overlap(0)): a plain launch; grid_dep_wait() is then a no-op.
+// A predecessor may thus still write this kernel's inputs while it already runs. The read-only path asks for data that
+// no one writes during the kernel, so what an earlier launch may have written is read by ordinary or L2 (__ldcg) loads:
+// no __ldg, and no `const T *__restrict__`, from which the compiler derives it and with it the right to load before the
+// wait. (Plain loads of the combine's rows cost 4-5 % of a layer of hidden 1024, __ldcg nothing.)
 extern int g_chain_overlap;
 template <class... KArgs, class... Args>
 inline cudaError_t launch_chain(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {

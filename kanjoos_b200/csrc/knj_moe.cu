@@ -198,8 +198,8 @@ int knj_moe_ffn_prefill_launch(const knj_moe_ffn_args *a, knj_stream_t s) {
   const PrefillWs w = carve_prefill(a->workspace, T, H, F, E, k);
   const int P = T * k;
 
-  // A chain of dependent launches: each but the router's for fewer than 32 tokens and the two of the fused combine's
-  // accumulator is prepared while its predecessor ends; what follows a memset (this one, the counting sort's) starts anew.
+  // A chain of dependent launches, each prepared while its predecessor ends, but for the row normalisation, the router of
+  // fewer than 32 tokens and the fused combine's accumulator; what follows a memset (this one, the counting sort's) starts anew.
   KNJ_CUDA(cudaMemsetAsync(w.status, 0, 16, as_stream(s)));  // the GEMMs raise it when a bounded wait gives up
   const void *src = a->x;
   int src_dt = a->x_dtype;

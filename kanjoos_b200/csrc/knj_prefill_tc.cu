@@ -776,7 +776,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
           if (!GATEUP && p.cmb_acc) {
             // the row's share of its token's weighted sum: one 16-byte reduction per lane (the k rows of a token
             // arrive from different CTAs in no fixed order)
-            const float w = __ldg(p.cmb_w + pr);
+            const float w = p.cmb_w[pr];
             float *dst = p.cmb_acc + (size_t)(pr / p.cmb_div) * p.N + m0 + mat * kRowsM + l16 * 4;
             asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(__uint_as_float(v.x) * w),
                          "f"(__uint_as_float(v.y) * w), "f"(__uint_as_float(v.z) * w), "f"(__uint_as_float(v.w) * w)
@@ -808,7 +808,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
 }
 
 // x (f32 / bf16 / f16) -> fp16 with saturation, rows dense
-__global__ void to_f16_kernel(const void *__restrict__ x, int dtype, int64_t ldx, int K, int64_t n, __half *__restrict__ out) {
+__global__ void to_f16_kernel(const void *x, int dtype, int64_t ldx, int K, int64_t n, __half *__restrict__ out) {
   grid_dep_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = i / K, c = i - r * K;
@@ -818,12 +818,12 @@ __global__ void to_f16_kernel(const void *__restrict__ x, int dtype, int64_t ldx
 }
 
 // the common case, bf16 rows whose length and stride are multiples of 8: 16 bytes in, 16 bytes out per thread and step
-__global__ void __launch_bounds__(256) bf16_to_f16_kernel(const uint4 *__restrict__ x, int64_t ldx8, int K8, int64_t n8,
+__global__ void __launch_bounds__(256) bf16_to_f16_kernel(const uint4 *x, int64_t ldx8, int K8, int64_t n8,
                                                           uint4 *__restrict__ out) {
   grid_dep_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = i / K8, c = i - r * K8;
-    const uint4 v = __ldg(x + r * ldx8 + c);
+    const uint4 v = __ldcg(x + r * ldx8 + c);
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     uint32_t o[4];
 #pragma unroll

@@ -313,3 +313,15 @@ def test_reference_device_unit_test_compiled_unmodified_against_this_library():
     fails = [ln for ln in out.splitlines() if "FAIL" in ln and "RESULT" not in ln]
     assert len(fails) == 1 and "dot label mismatch" in fails[0], fails
     assert 'expected: "asm(v_dot4_i32_i8)", got: "intrinsic(dp4a)"' in out
+
+
+def test_chained_kernels_do_not_take_read_only_inputs():
+    """A kernel launched through launch_chain may run while its predecessor still writes its inputs, so none may be
+    declared `const T *__restrict__` (the read-only path wants data nobody writes during the kernel)."""
+    src = os.path.join(ROOT, "kanjoos_b200", "csrc")
+    text = "\n".join(open(os.path.join(src, f)).read() for f in sorted(os.listdir(src)) if f.endswith((".cu", ".cuh")))
+    chained = set(re.findall(r"launch_chain\((\w+_kernel)", text))
+    assert {"router_topk_kernel", "permute_kernel", "combine_kernel", "to_f16_kernel"} <= chained
+    for name in chained:
+        params = re.search(r"__global__[^;{]*?\b" + name + r"\s*\(([^)]*)\)\s*\{", text).group(1)
+        assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", params), f"{name}({params})"
