@@ -383,11 +383,12 @@ __global__ void __launch_bounds__(256) permute_kernel(const int32_t *pair_exp, i
   __shared__ int wsum[8];
   int32_t *row = pair_idx + (size_t)e * idx_stride;
   int base = 0;  // identical in every thread
+  const bool wide = (reinterpret_cast<uintptr_t>(pair_exp) & 15u) == 0;  // a caller's tap array may start anywhere
   // eight consecutive pairs per thread and pass: count, block-wide exclusive scan, write in order
   for (int p0 = 0; p0 < P; p0 += 2048) {
     const int first = p0 + threadIdx.x * 8;
     int v[8];
-    if (first + 8 <= P && (P & 3) == 0) {
+    if (wide && first + 8 <= P) {
       const int4 a = __ldcg(reinterpret_cast<const int4 *>(pair_exp + first));
       const int4 b = __ldcg(reinterpret_cast<const int4 *>(pair_exp + first) + 1);
       v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;

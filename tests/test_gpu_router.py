@@ -83,6 +83,19 @@ def test_permute_tables(T, E, k):
     assert n_active[1] == hist.max()
 
 
+@pytest.mark.parametrize("P,off", [(64, 0), (64, 1), (67, 0), (67, 3), (4096, 2)])
+def test_permute_tables_of_an_unaligned_pair_list(P, off):
+    """The pair list may be a caller's array that starts at any element."""
+    from kanjoos_b200 import ops
+    E = 16
+    pe = np.random.Generator(np.random.Philox([P, off])).integers(0, E, size=P + off, dtype=np.int32)
+    pair_idx, pair_cnt, _, _ = ops.moe_permute(dev(pe)[off:], E, P)
+    pair_idx, pair_cnt = pair_idx.cpu().numpy(), pair_cnt.cpu().numpy()
+    for e in range(E):
+        want = np.nonzero(pe[off:] == e)[0]
+        assert pair_cnt[e] == len(want) and np.array_equal(pair_idx[e, :len(want)], want) and (pair_idx[e, len(want):] == -1).all()
+
+
 @pytest.mark.parametrize("T,E,dtype", [(32, 128, "f32"), (1183, 128, "bf16"), (1185, 128, "bf16"), (1185, 128, "f32"),
                                        (77, 40, "bf16"), (4737, 128, "bf16")])
 def test_router_logits_do_not_depend_on_the_tile(T, E, dtype):
