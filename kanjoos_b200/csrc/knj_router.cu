@@ -134,7 +134,8 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 // CTA = 4 warps; K in steps of 32 through a cp.async pipeline of NSTAGE stages (activation tile + router tile per stage).
 // Every logit is one chain of f32 additions in ascending K whatever the tile, so that near-ties of the routing fall the
-// same way at every token count (K split over warps was faster still, 9 us at 100 and 512 tokens, but changed the sums'
+// same way at every token count from 32 on (below, or with unaligned rows, router_logits_kernel adds in another order;
+// K split over warps was faster still, 9 us at 100 and 512 tokens, but changed the sums'
 // order: one near-tie in 16384 tokens fell the other way).
 // MT = 64: 64 tokens x 64 experts, a warp 16 tokens x 64 experts. MT = 16: 16 tokens x 32 experts, a warp 16 tokens x 8.
 // Both are bound by a step's latency over the steps in flight: 64-token tiles with three stages took 36 us for 100 f32
