@@ -567,10 +567,11 @@ def run_gpu(args):
             dec = decode_section(torch, max(5, args.steps), args.warmup, pk)
 
     # kernels of this library per layer step: router logits + top-k, permutation (count, scan, scatter for
-    # P >= 8192, else one kernel) + active list, to_f16, gate+up, down, then combine (N = 1) or the exchange kernels
+    # P >= 8192, else one kernel; the exchange forms also list the active experts), to_f16, gate+up, down, then combine
+    # (N = 1) or the exchange kernels
     n_perm = 4 if T * TOPK >= 8192 else 2
     if world == 1:
-        launches = 2 + n_perm + 1 + 2 + 1
+        launches = 2 + (n_perm - 1) + 1 + 2 + 1
     elif args.exchange == "peer":
         # rows to fp16, router (2), table stores, arrival, wait, local expert ids, plan, gate+up, down, partial sums to
         # the owners, arrival, wait, rank reduce (the rows themselves travel as copy-engine copies, not kernels)
