@@ -9,7 +9,7 @@
 // row tiles, CTAs 2i and 2i+1 form a cluster and share one cta_group::2 MMA
 // (M = 256 over the pair, each CTA gathers half of the bucket's token rows):
 //   warps 0..15 unpackers: per superblock the eight (d*sc, -dmin*m) pairs of a
-//               weight row are formed in fp16 (exact), per slab each thread turns
+//               weight row are formed in fp16, per slab each thread turns
 //               16 code bytes of one matrix into 32 fp16 weights and stores them
 //               into the K-major 128-byte-swizzled operand tile or, for a bucket
 //               of up to 128 tokens, into the half of tensor memory that its
@@ -31,10 +31,13 @@
 // Gate and up share the token operand: two accumulators (TMEM columns [0,256)
 // and [256,512)) are fed from two weight tiles per slab.
 //
-// Precision. Operands are fp16, not bf16: a Q4_K weight rounded to fp16 is off
-// by <= 2^-12 relative, which keeps the layer's relative RMSE well inside the
-// 1e-3 budget of the tensor-core path; bf16 operands (2^-9) would not. The
-// activations are converted to fp16 beforehand with a saturating convert, and
+// Precision. Operands are fp16, not bf16. A Q4_K weight carries three fp16
+// roundings: of d*sc, of dmin*m (products of up to 17 bits) and of the fused
+// q*(d*sc) - dmin*m, whose terms cancel. For centred weights (d about 1.2e-4,
+// dmin = 7.5 d) that is 5.5e-4 of the weights' RMS, 2.1e-4 of it the last
+// rounding alone; the layer is off by 9.8e-4 relative (512 tokens, hidden 2048,
+// against float64), just inside the 1e-3 budget of the tensor-core path. bf16
+// operands, three bits shorter, would not be. The activations are converted to fp16 beforehand with a saturating convert, and
 // the SiLU*up intermediate is stored as fp16 after a fixed 2^-6 prescale
 // (undone in the down epilogue), which holds magnitudes up to 4.1e6.
 //
@@ -555,8 +558,8 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
       const uint8_t *raw = smem + off_raw + buf * S::kRawBuf + (mat * kRowsM + row) * KNJ_Q4K_BYTES;
 
       // ---- once per superblock: (d*sc, -dmin*m) of this row's eight sub-blocks in fp16.
-      // d*sc is an 11-bit by 6-bit product, so one fp16 multiply rounds it exactly as a
-      // float multiply followed by a conversion would.
+      // d*sc is an 11-bit by 6-bit product: the fp16 multiply rounds it once, as a float
+      // multiply (exact) followed by a conversion would.
       const __half2 k1024 = __float2half2_rn(1024.0f);
       __half2 d1h[4 * kPar], m1h[4 * kPar];
       {
