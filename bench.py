@@ -521,10 +521,10 @@ def run_gpu(args):
         t_tensor = flops / (pk["bf16_tflops"] * 1e12)
         assert int(status.item()) == 0, "a bounded wait inside the grouped GEMM gave up"
         # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum of this kernel) as ncu counted them on
-        # this workload in a one-pass capture of the same command: at T=16384 532.3 + 184.3 MB, at T=4096
-        # 261.5 + 38.7 MB (uniform router, N=1); other sizes have no capture
+        # this workload in a one-pass capture of the same command: at T=16384 531.2 + 183.4 MB, at T=4096
+        # 260.6 + 38.5 MB (uniform router, N=1); other sizes have no capture
         w_bytes = int((pair_cnt > 0).sum().item()) * 2 * F * (H // 256) * 144
-        measured = {(16384, "uniform"): 716.6e6, (4096, "uniform"): 300.2e6}
+        measured = {(16384, "uniform"): 714.6e6, (4096, "uniform"): 299.2e6}
         traffic = measured.get((T, args.routing)) if world == 1 else None
         traffic_note = ("ncu one-pass DRAM counters of this kernel on this workload; algorithmic bytes (weights once + fp16 rows "
                         "in + fp16 rows out) = %.1f MB" % ((w_bytes + rows // TOPK * H * 2 + rows * F * 2) / 1e6)) if traffic else None
