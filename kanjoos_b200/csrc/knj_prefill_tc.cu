@@ -549,7 +549,8 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_grouped_tc_kernel(const __gri
     const int mat = NMAT == 2 ? tid >> 8 : 0, par0 = NMAT == 2 ? 0 : tid >> 8;
     auto unpack = [&](auto ta) {
     // few tokens: the unpackers set the pace, so the weights are formed before the stage is waited for; full buckets
-    // wait for the tensor pipe, and holding formed weights back there was slower (1.96 against 1.89 ms at 16384 tokens)
+    // wait for the tensor pipe, and holding formed weights back there was slower (1.96 against 1.89 ms at 16384 tokens, measured with eight
+    // unpacker warps and cp.async rows)
     constexpr bool kEarly = decltype(ta)::value;
     int buf = 0, stage = 0;
     uint32_t raw_par = 0, empty_par = 1;             // a fresh barrier passes a wait for parity 1
