@@ -271,16 +271,12 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const float *logits, i
   const int t = blockIdx.x * 4 + (threadIdx.x >> 5);
   grid_dep_wait();
   if (t >= T) return;
-  int sel_e[8];
-  float sel_w[8];
-  warp_topk(logits + (size_t)t * E, E, k, lane, sel_e, sel_w);
-  if (lane == 0) {
-#pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      if (s >= k) break;
-      pair_exp[(size_t)t * k + s] = sel_e[s];
-      pair_w[(size_t)t * k + s] = sel_w[s];
-    }
+  int e;
+  float w;
+  warp_topk(logits + (size_t)t * E, E, k, lane, e, w);
+  if (lane < k) {
+    pair_exp[(size_t)t * k + lane] = e;
+    pair_w[(size_t)t * k + lane] = w;
   }
 }
 
@@ -712,16 +708,12 @@ __global__ void __launch_bounds__(256) moe_front_kernel(const FrontParams p) {
   {
     const int t = t0 + warp;
     if (warp < p.tpc && t < p.T) {
-      int sel_e[8];
-      float sel_w[8];
-      warp_topk(p.logits + (size_t)t * p.E, p.E, p.k, lane, sel_e, sel_w);
-      if (lane == 0) {
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-          if (s >= p.k) break;
-          p.pair_exp[(size_t)t * p.k + s] = sel_e[s];
-          p.pair_w[(size_t)t * p.k + s] = sel_w[s];
-        }
+      int e;
+      float w;
+      warp_topk(p.logits + (size_t)t * p.E, p.E, p.k, lane, e, w);
+      if (lane < p.k) {
+        p.pair_exp[(size_t)t * p.k + lane] = e;
+        p.pair_w[(size_t)t * p.k + lane] = w;
       }
     }
   }

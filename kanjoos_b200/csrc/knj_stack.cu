@@ -28,6 +28,7 @@
 #include "knj_topk.cuh"
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 using namespace knj;
@@ -85,10 +86,7 @@ __device__ __forceinline__ void red_release(unsigned *p, unsigned v) {
 // times in total; false: a wait ran out (here or elsewhere).
 __device__ __forceinline__ void grid_arrive(unsigned *sync) {
   __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    red_release(sync, 1u);
-  }
+  if (threadIdx.x == 0) red_release(sync, 1u);  // cumulative: releases what the CTA barrier ordered before it
 }
 __device__ __forceinline__ bool grid_wait(unsigned *sync, unsigned target, long long limit) {
   int ok = 1;
@@ -182,11 +180,14 @@ __device__ __noinline__ void stage_logits(const StackParams &p, const LayerDesc 
       if (has_norm) nraw[q] = __ldg(reinterpret_cast<const uint4 *>(L.norm_w + 8 * ch));
     }
   }
+  // the token rows as asynchronous copies (through L2): all under way at once and no registers held (a loop of load and
+  // store cost up to eight trips to L2)
   for (int i = threadIdx.x; i < nt * cpr; i += kThreads) {
     const int r = i / cpr, ch = i - r * cpr;
-    *reinterpret_cast<uint4 *>(rows_s + (size_t)r * row_bytes + 16 * ch) =
-        __ldcg(reinterpret_cast<const uint4 *>(static_cast<const uint8_t *>(L.x) + (int64_t)(tg * 8 + r) * L.ldx * esz + 16 * ch));
+    const uint8_t *src = static_cast<const uint8_t *>(L.x) + (int64_t)(tg * 8 + r) * L.ldx * esz + 16 * ch;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(rows_s + (size_t)16 * i)), "l"(src) : "memory");
   }
+  asm volatile("cp.async.commit_group;" ::: "memory");
 #pragma unroll
   for (int q = 0; q < kPer; ++q) {
     const int i = threadIdx.x + q * kThreads;
@@ -206,6 +207,7 @@ __device__ __noinline__ void stage_logits(const StackParams &p, const LayerDesc 
       *reinterpret_cast<float4 *>(wr_s + (size_t)8 * i + 4) = make_float4(v[4], v[5], v[6], v[7]);
     }
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
   KNJ_STAMP(11);
   const int es = warp % epi, tpw = max(1, epi / 2);
@@ -276,22 +278,34 @@ __device__ __noinline__ void stage_plan(const StackParams &p, const LayerDesc &L
   unsigned char *ord = smem + pl.ord;
     for (int t = threadIdx.x; t < T; t += kThreads) scale_s[t] = __ldcg(p.scales + t);
     for (int a = threadIdx.x; a < 256; a += kThreads) mask[a] = 0ull;
-    for (int t = warp; t < T; t += q4e::kWarps) {
-      int se[8];
-      float sw[8];
-      if (E <= 128) warp_topk<4>(p.logits + (size_t)t * E, E, k, lane, se, sw);
-      else warp_topk(p.logits + (size_t)t * E, E, k, lane, se, sw);
-      if (lane == 0) {
+    auto select = [&](auto epl, auto group) {  // tokens warp, warp + 16, ...: `group` of them at a time
+      constexpr int kEpl = decltype(epl)::value, kNt = decltype(group)::value;
+#pragma unroll 1
+      for (int t0 = warp; t0 < T; t0 += q4e::kWarps * kNt) {
+        float v[kNt][kEpl], w[kNt];
+        int e[kNt];
 #pragma unroll
-        for (int s = 0; s < 8; ++s) {
-          if (s >= k) break;
-          sel_e[t * k + s] = se[s];
-          sel_w[t * k + s] = sw[s];
-          if (c == 0 && L.tap_exp) L.tap_exp[t * k + s] = se[s];
-          if (c == 0 && L.tap_w) L.tap_w[t * k + s] = sw[s];
+        for (int n = 0; n < kNt; ++n) topk_load<kEpl>(p.logits + (size_t)min(t0 + q4e::kWarps * n, T - 1) * E, E, lane, v[n]);
+        warp_topk<kEpl, kNt>(v, k, lane, e, w);
+#pragma unroll
+        for (int n = 0; n < kNt; ++n) {
+          const int t = t0 + q4e::kWarps * n;
+          if (t < T && lane < k) {
+            sel_e[t * k + lane] = e[n];
+            sel_w[t * k + lane] = w[n];
+            if (c == 0 && L.tap_exp) L.tap_exp[t * k + lane] = e[n];
+            if (c == 0 && L.tap_w) L.tap_w[t * k + lane] = w[n];
+          }
         }
       }
-    }
+    };
+    using std::integral_constant;
+    // A token alone is latency (1.8 us), so a warp's tokens go together: two up to 32 tokens, four above (a layer of 64
+    // tokens 2 us shorter than one after the other); a second and fourth token that do not exist repeat the last one.
+    if (E > 128) select(integral_constant<int, kMaxEPerLane>{}, integral_constant<int, 1>{});
+    else if (T <= q4e::kWarps) select(integral_constant<int, 4>{}, integral_constant<int, 1>{});
+    else if (T <= 2 * q4e::kWarps) select(integral_constant<int, 4>{}, integral_constant<int, 2>{});
+    else select(integral_constant<int, 4>{}, integral_constant<int, 4>{});
     __syncthreads();
     for (int pr = threadIdx.x; pr < P; pr += kThreads) {
       const int t = pr / k, e = sel_e[pr];

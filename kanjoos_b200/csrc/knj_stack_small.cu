@@ -83,8 +83,7 @@ __device__ __forceinline__ void red_release(unsigned *p, unsigned v) {
 __device__ __forceinline__ void grid_arrive(unsigned *sync) {
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();
-    red_release(sync, 1u);
+    red_release(sync, 1u);  // cumulative: releases what the CTA barrier ordered before it
   }
 }
 __device__ __forceinline__ bool grid_wait(unsigned *sync, unsigned target, long long limit) {
@@ -468,19 +467,14 @@ __global__ void __launch_bounds__(kThreads, 1) moe_stack_small_kernel(const Stac
 
     // ---- top-k per token (every CTA for itself), then the distinct experts in ascending order
     if (warp < T) {
-      int se[8];
-      float sw[8];
-      if (E <= 128) warp_topk<4>(p.logits + (size_t)warp * E, E, k, lane, se, sw);
-      else warp_topk(p.logits + (size_t)warp * E, E, k, lane, se, sw);
-      if (lane == 0) {
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-          if (s >= k) break;
-          sel_e[warp * k + s] = se[s];
-          sel_w[warp * k + s] = sw[s];
-          if (c == 0 && L.tap_exp) L.tap_exp[warp * k + s] = se[s];
-          if (c == 0 && L.tap_w) L.tap_w[warp * k + s] = sw[s];
-        }
+      int e;
+      float w;
+      warp_topk(p.logits + (size_t)warp * E, E, k, lane, e, w);
+      if (lane < k) {
+        sel_e[warp * k + lane] = e;
+        sel_w[warp * k + lane] = w;
+        if (c == 0 && L.tap_exp) L.tap_exp[warp * k + lane] = e;
+        if (c == 0 && L.tap_w) L.tap_w[warp * k + lane] = w;
       }
     }
     if (warp == kWarps - 1 && lane < 8) bitmap[lane] = 0u;

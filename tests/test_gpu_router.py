@@ -113,3 +113,19 @@ def test_router_logits_do_not_depend_on_the_tile(T, E, dtype):
     want = x.double() @ bf16_dev(wr).double().T
     # f32 sums of 2048 exact products: the error of a sum is below sqrt(2048) * 2^-24 of its terms' 2-norm, 3e-6
     assert report(logits.cpu().numpy(), want.float().cpu().numpy(), f"router logits {T}x{E}")["rel_rmse"] <= 1e-5
+
+
+@pytest.mark.parametrize("E", [33, 128, 129, 256])
+def test_topk_of_equal_logits(E):
+    """Ties inside a lane (ids 32 apart) and across lanes: value descending, id ascending. A zero row's logits are the
+    biases themselves, so the order is known exactly; the weights carry one expf and two divisions (1e-6)."""
+    from kanjoos_b200 import ops
+    k, T, H = 8, 6, 256
+    rng = np.random.Generator(np.random.Philox(E))
+    for case in range(4):
+        bias = [np.zeros(E), np.arange(E) // 32 * 0.5, rng.integers(0, 3, E) * 0.25, -(np.arange(E) % 7) * 1.0][case].astype(np.float32)
+        _, pe, pw = ops.router_topk(torch.zeros((T, H), device="cuda"), torch.zeros((E, H), dtype=torch.bfloat16, device="cuda"), k, dev(bias))
+        want = np.argsort(-bias, kind="stable")[:k]
+        assert (pe.view(T, k).cpu().numpy() == want[None]).all(), case
+        w = np.exp(bias[want].astype(np.float64))
+        assert np.abs(pw.view(T, k).cpu().numpy() - (w / w.sum())[None]).max() < 1e-6

@@ -45,6 +45,22 @@ def test_single_layer_f32_against_cpu_path(T, E, H, F, k):
     st.close()
 
 
+@pytest.mark.parametrize("T,E", [(16, 128), (17, 128), (32, 128), (33, 100), (48, 128), (61, 128), (33, 160)])
+def test_routing_is_the_layer_launch_s_at_every_group_of_tokens(T, E):
+    """The stack's plan selects one, two or four tokens per warp at a time (and one from 129 experts on): the same
+    experts and the same bits of the weights as the layer launch, whose front kernel takes one."""
+    from kanjoos_b200.moe import FusedMoeStack, MoeFfnLayer
+    H, F, k = 512, 256, 8
+    banks, _ = _banks(806, 1, E, H, F)
+    x = dev(synth.hidden_rows(806, T, H))
+    st = FusedMoeStack(banks, top_k=k, n_tokens=T, dtype=torch.float32, residual=False, taps=True)
+    st.step(x)
+    st.status()
+    _, pe, pw = MoeFfnLayer(banks[0], top_k=k, max_tokens=T, residual=False).decode(x, return_routing=True)
+    assert torch.equal(pe, st.taps[0][0]) and torch.equal(pw.view(torch.int32), st.taps[0][1].view(torch.int32))
+    st.close()
+
+
 def test_stack_follows_layer_by_layer_launches():
     from kanjoos_b200.moe import FusedMoeStack, MoeStack
     L, E, H, F, k, T = 6, 32, 1024, 512, 8, 2
