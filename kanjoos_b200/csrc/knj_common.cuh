@@ -42,6 +42,11 @@ int sm_count();  // SMs of the current device (cached per device)
 // The permutation tables without the active-expert list (knj_router.cu).
 int moe_permute_tables(const int32_t *pair_exp, int P, int E, int idx_stride, int32_t *pair_idx, int32_t *pair_cnt, void *scratch,
                        size_t scratch_bytes, cudaStream_t st);
+// knj_moe_front_launch that clears `clear_bytes` bytes from `counter` on (0: its own counters only), so that a caller with
+// other words to clear behind them needs no fill of its own in front of the launch.
+int moe_front(const void *x, int x_dtype, int64_t ldx, const uint16_t *norm_w, float eps, const uint16_t *Wr_bf16, const float *bias, int T,
+              int H, int E, int k, float *logits, int32_t *pair_exp, float *pair_w, int32_t *pair_idx, int idx_stride, int32_t *pair_cnt,
+              int32_t *exp_list, int32_t *n_active, float *xn, uint32_t *counter, size_t clear_bytes, knj_stream_t s);
 // knj_ep_combine_partial_peer_launch with every owner's array entered at element `parts_off`; with `stage` (f32
 // [T][H], local) the rows of other ranks' tokens are written there instead, one dense block per owner
 int ep_combine_partial_peer_at(const float *Y, const int32_t *pair_exp, const float *pair_w, int T, int H, int k, int exp_lo, int exp_hi,

@@ -860,6 +860,43 @@ int moe_permute_tables(const int32_t *pair_exp, int P, int E, int idx_stride, in
 }
 }  // namespace knj
 
+#ifdef KNJ_TRACE
+static unsigned long long *g_front_trace = nullptr;
+#endif
+namespace knj {
+int moe_front(const void *x, int x_dtype, int64_t ldx, const uint16_t *norm_w, float eps, const uint16_t *Wr_bf16, const float *bias, int T,
+              int H, int E, int k, float *logits, int32_t *pair_exp, float *pair_w, int32_t *pair_idx, int idx_stride, int32_t *pair_cnt,
+              int32_t *exp_list, int32_t *n_active, float *xn, uint32_t *counter, size_t clear_bytes, knj_stream_t s) {
+  KNJ_REQUIRE(x && Wr_bf16 && logits && pair_exp && pair_w && pair_idx && pair_cnt && exp_list && n_active && xn && counter,
+              "knj_moe_front: null pointer");
+  KNJ_REQUIRE(T >= 1 && T <= kFrontMaxT, "knj_moe_front: T=%d out of range (1..%d)", T, kFrontMaxT);
+  KNJ_REQUIRE(H % 256 == 0 && H <= 256 * kFrontMaxSlices, "knj_moe_front: H=%d must be a multiple of 256, <= %d", H,
+              256 * kFrontMaxSlices);
+  KNJ_REQUIRE(E >= 1 && E <= 256 && k >= 1 && k <= 8 && k <= E && idx_stride >= T, "knj_moe_front: bad E / k / stride");
+  KNJ_REQUIRE(aligned16(Wr_bf16) && aligned16(xn) && (!norm_w || aligned16(norm_w)) && aligned16(x) && ldx % 8 == 0,
+              "knj_moe_front: 16-byte alignment of x rows, weights and normalised rows");
+  FrontParams p{};
+  p.x = x; p.x_dtype = x_dtype; p.ldx = ldx; p.norm_w = reinterpret_cast<const __nv_bfloat16 *>(norm_w); p.eps = eps;
+  p.Wr = reinterpret_cast<const __nv_bfloat16 *>(Wr_bf16); p.bias = bias; p.T = T; p.H = H; p.E = E; p.k = k;
+  p.idx_stride = idx_stride; p.logits = logits; p.pair_exp = pair_exp; p.pair_w = pair_w; p.pair_idx = pair_idx;
+  p.pair_cnt = pair_cnt; p.exp_list = exp_list; p.n_active = n_active; p.xn = xn;
+  p.counter = counter;
+#ifdef KNJ_TRACE
+  p.trace = g_front_trace;
+#endif
+  p.tpc = (T + 7) / 8;  // eight token groups at most: ~128 CTAs at every batch, and the serial walk over a CTA's tokens stays short
+  const int n_tg = (T + p.tpc - 1) / p.tpc;
+  KNJ_CUDA(cudaMemsetAsync(counter, 0, clear_bytes ? clear_bytes : sizeof(uint32_t) * (1 + n_tg), as_stream(s)));
+  dim3 grid((E + 7) / 8, n_tg);
+  cudaError_t le;
+  if (x_dtype == KNJ_DT_F32) le = launch_chain(moe_front_kernel<KNJ_DT_F32>, grid, dim3(256), 0, as_stream(s), p);
+  else if (x_dtype == KNJ_DT_BF16) le = launch_chain(moe_front_kernel<KNJ_DT_BF16>, grid, dim3(256), 0, as_stream(s), p);
+  else le = launch_chain(moe_front_kernel<KNJ_DT_F16>, grid, dim3(256), 0, as_stream(s), p);
+  KNJ_CUDA(le);
+  return launch_status("moe_front_kernel");
+}
+}  // namespace knj
+
 extern "C" {
 
 int knj_rmsnorm_launch(const void *x, int x_dtype, int64_t ldx, const uint16_t *w_bf16, float eps, int T, int H,
@@ -926,7 +963,6 @@ int knj_moe_permute_launch(const int32_t *pair_exp, int P, int E, int idx_stride
 }
 
 #ifdef KNJ_TRACE
-static unsigned long long *g_front_trace = nullptr;
 // measurement builds only: device buffer of 16 u64 that receives global-timer stamps of the front kernel's phases
 void knj_trace_front(void *dev_buf) { g_front_trace = static_cast<unsigned long long *>(dev_buf); }
 #endif
@@ -935,33 +971,8 @@ int knj_moe_front_launch(const void *x, int x_dtype, int64_t ldx, const uint16_t
                          const uint16_t *Wr_bf16, const float *bias, int T, int H, int E, int k, float *logits,
                          int32_t *pair_exp, float *pair_w, int32_t *pair_idx, int idx_stride, int32_t *pair_cnt,
                          int32_t *exp_list, int32_t *n_active, float *xn, uint32_t *counter, knj_stream_t s) {
-  KNJ_REQUIRE(x && Wr_bf16 && logits && pair_exp && pair_w && pair_idx && pair_cnt && exp_list && n_active && xn && counter,
-              "knj_moe_front: null pointer");
-  KNJ_REQUIRE(T >= 1 && T <= kFrontMaxT, "knj_moe_front: T=%d out of range (1..%d)", T, kFrontMaxT);
-  KNJ_REQUIRE(H % 256 == 0 && H <= 256 * kFrontMaxSlices, "knj_moe_front: H=%d must be a multiple of 256, <= %d", H,
-              256 * kFrontMaxSlices);
-  KNJ_REQUIRE(E >= 1 && E <= 256 && k >= 1 && k <= 8 && k <= E && idx_stride >= T, "knj_moe_front: bad E / k / stride");
-  KNJ_REQUIRE(aligned16(Wr_bf16) && aligned16(xn) && (!norm_w || aligned16(norm_w)) && aligned16(x) && ldx % 8 == 0,
-              "knj_moe_front: 16-byte alignment of x rows, weights and normalised rows");
-  FrontParams p{};
-  p.x = x; p.x_dtype = x_dtype; p.ldx = ldx; p.norm_w = reinterpret_cast<const __nv_bfloat16 *>(norm_w); p.eps = eps;
-  p.Wr = reinterpret_cast<const __nv_bfloat16 *>(Wr_bf16); p.bias = bias; p.T = T; p.H = H; p.E = E; p.k = k;
-  p.idx_stride = idx_stride; p.logits = logits; p.pair_exp = pair_exp; p.pair_w = pair_w; p.pair_idx = pair_idx;
-  p.pair_cnt = pair_cnt; p.exp_list = exp_list; p.n_active = n_active; p.xn = xn;
-  p.counter = counter;
-#ifdef KNJ_TRACE
-  p.trace = g_front_trace;
-#endif
-  p.tpc = (T + 7) / 8;  // eight token groups at most: ~128 CTAs at every batch, and the serial walk over a CTA's tokens stays short
-  const int n_tg = (T + p.tpc - 1) / p.tpc;
-  KNJ_CUDA(cudaMemsetAsync(counter, 0, sizeof(uint32_t) * (1 + n_tg), as_stream(s)));
-  dim3 grid((E + 7) / 8, n_tg);
-  cudaError_t le;
-  if (x_dtype == KNJ_DT_F32) le = launch_chain(moe_front_kernel<KNJ_DT_F32>, grid, dim3(256), 0, as_stream(s), p);
-  else if (x_dtype == KNJ_DT_BF16) le = launch_chain(moe_front_kernel<KNJ_DT_BF16>, grid, dim3(256), 0, as_stream(s), p);
-  else le = launch_chain(moe_front_kernel<KNJ_DT_F16>, grid, dim3(256), 0, as_stream(s), p);
-  KNJ_CUDA(le);
-  return launch_status("moe_front_kernel");
+  return moe_front(x, x_dtype, ldx, norm_w, eps, Wr_bf16, bias, T, H, E, k, logits, pair_exp, pair_w, pair_idx, idx_stride, pair_cnt,
+                   exp_list, n_active, xn, counter, 0, s);
 }
 
 int knj_active_list_launch(const int32_t *pair_cnt, int E, int32_t *exp_list, int32_t *n_active, knj_stream_t s) {
