@@ -15,6 +15,8 @@
 //     products and the f32 accumulation of mma.sync are exact to f32 level; the
 //     two planes of a token sit in adjacent MMA columns, so one m16n8k16 covers
 //     four tokens and the planes are summed in-thread;
+//     (activations that are 16-bit to begin with fit one plane exactly; a dense product of such rows puts eight of them in
+//     the eight columns, PL = 1 below: the same weights are then unpacked half as often);
 //   * the min term is one more MMA per superblock: A = the eight 6-bit m_sb,
 //     B = the per-32 sums of the token's planes.
 //
@@ -53,7 +55,10 @@ constexpr int kJobTok = 4;                              // tokens of one job = o
 // sub-block's plane); inside a unit, 16 bytes per (plane, t) at 16 * (4 * plane + t): the eight lanes of a
 // quarter-warp (planes 0/1 of one token, t = 0..3) read one unit without bank conflicts. Then the per-32
 // sums / 64 as fp16 pairs (sub-blocks 2t, 2t+1): high plane at 1024 + 4t, low plane at 1040 + 4t.
+// With one plane (PL = 1) a slot holds two tokens, the second in the low plane's place; the low plane of its sums then
+// lies 32 bytes behind the high one.
 constexpr int kPanelBytes = 1088;
+template <int PL> __host__ __device__ constexpr int job_tokens() { return PL == 1 ? 2 * kJobTok : kJobTok; }
 
 __device__ __forceinline__ uint32_t mul_f16x2(uint32_t a, uint32_t b) {
   uint32_t d;
@@ -103,7 +108,9 @@ __device__ __forceinline__ void load8_f32(const void *base, int dtype, int64_t e
 
 // One warp converts the 256 values of one (token, superblock) -- lane l holds values 8l..8l+7 -- into the panel
 // at `dst`; returns 1 / scale (the same in every lane).
-__device__ __forceinline__ float panel_convert(const float (&v)[8], uint8_t *dst, int lane) {
+// With one plane: `odd` = the slot's second token.
+template <int PL = 2>
+__device__ __forceinline__ float panel_convert(const float (&v)[8], uint8_t *dst, int lane, int odd = 0) {
   float amax = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
@@ -123,8 +130,8 @@ __device__ __forceinline__ float panel_convert(const float (&v)[8], uint8_t *dst
       const float f = v[4 * q + i] * s;
       hh[i] = __float2half_rn(f);
       const float hf = __half2float(hh[i]);
-      ll[i] = __float2half_rn(f - hf);
-      part += hf + __half2float(ll[i]);
+      ll[i] = __float2half_rn(f - hf);  // one plane: nothing is left (16-bit values, scaled by a power of two)
+      part += PL == 2 ? hf + __half2float(ll[i]) : hf;
     }
     hw[2 * q] = pack_h2(hh[0], hh[2]);
     hw[2 * q + 1] = pack_h2(hh[1], hh[3]);
@@ -132,16 +139,17 @@ __device__ __forceinline__ float panel_convert(const float (&v)[8], uint8_t *dst
     lw[2 * q + 1] = pack_h2(ll[1], ll[3]);
   }
   const int sb = lane >> 2, t = sb >> 1, u = 4 * (sb & 1) + (lane & 3);
-  *reinterpret_cast<uint4 *>(dst + 128 * u + 16 * t) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-  *reinterpret_cast<uint4 *>(dst + 128 * u + 16 * (4 + t)) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+  *reinterpret_cast<uint4 *>(dst + 128 * u + 16 * ((PL == 1 ? 4 * odd : 0) + t)) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+  if (PL == 2) *reinterpret_cast<uint4 *>(dst + 128 * u + 16 * (4 + t)) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
   part += __shfl_xor_sync(0xffffffffu, part, 1);
   part += __shfl_xor_sync(0xffffffffu, part, 2);              // the sub-block's sum, in its four lanes
   const float next = __shfl_down_sync(0xffffffffu, part, 4);  // the following sub-block's
   if ((lane & 7) == 0) {
     const float s0 = part * 0.015625f, s1 = next * 0.015625f;  // |sum| < 32 * 2^14: / 64 keeps it inside fp16
     const __half h0 = __float2half_rn(s0), h1 = __float2half_rn(s1);
-    *reinterpret_cast<uint32_t *>(dst + 1024 + 4 * t) = pack_h2(h0, h1);
-    *reinterpret_cast<uint32_t *>(dst + 1040 + 4 * t) =
+    uint8_t *sums = dst + 1024 + (PL == 1 ? 16 * odd : 0) + 4 * t;
+    *reinterpret_cast<uint32_t *>(sums) = pack_h2(h0, h1);
+    *reinterpret_cast<uint32_t *>(sums + (PL == 1 ? 32 : 16)) =
         pack_h2(__float2half_rn(s0 - __half2float(h0)), __float2half_rn(s1 - __half2float(h1)));
   }
   return __uint_as_float((uint32_t)(127 - e) << 23);
@@ -171,9 +179,11 @@ __device__ __forceinline__ void header_pairs(const uint4 &hd, uint32_t sel16, bo
 // (see tile_row) and receives, per group q, the superblock's contribution to (row wrow, token 4q + t) in
 // rg[q] and to (row wrow + 8, token 4q + t) in rh[q], in the units of the token's scaled planes; the caller
 // multiplies by 1 / scale. after_loads() runs once the weights are in registers (the stage may be refilled).
-template <int NG, class AfterLoads>
+// One plane (PL = 1, NG = 1): the two columns of a lane are tokens 2t and 2t + 1 of the job, in rg[0 / 1] and rh[0 / 1].
+template <int NG, int PL = 2, class AfterLoads>
 __device__ __forceinline__ void tile_part(const uint8_t *stage, int pitch, int wrow, const uint8_t *pan, int tok_stride,
-                                          int lane, float (&rg)[NG], float (&rh)[NG], AfterLoads after_loads) {
+                                          int lane, float (&rg)[PL == 1 ? 2 : NG], float (&rh)[PL == 1 ? 2 : NG], AfterLoads after_loads) {
+  static_assert(PL == 2 || NG == 1, "one plane: one column group");
   const int g = lane >> 2, t = lane & 3;
   const uint8_t *wg_row = stage + wrow * pitch, *wh_row = stage + (wrow + 8) * pitch;
   const uint4 hg = *reinterpret_cast<const uint4 *>(wg_row), hh = *reinterpret_cast<const uint4 *>(wh_row);
@@ -210,7 +220,12 @@ __device__ __forceinline__ void tile_part(const uint8_t *stage, int pitch, int w
 #pragma unroll
   for (int q = 0; q < NG; ++q) {
     const uint32_t sx = *reinterpret_cast<const uint32_t *>(col + q * grp_stride + 1024 + 16 * (g & 1) + 4 * t);
-    mma_f16_16816_zero(cm[q], mmg, mmh, 0u, 0u, sx, 0u);
+    if (PL == 1) {  // both planes of the sums, along K
+      const uint32_t sl = *reinterpret_cast<const uint32_t *>(col + 1056 + 16 * (g & 1) + 4 * t);
+      mma_f16_16816_zero(cm[q], mmg, mmh, mmg, mmh, sx, sl);
+    } else {
+      mma_f16_16816_zero(cm[q], mmg, mmh, 0u, 0u, sx, 0u);
+    }
 #pragma unroll
     for (int c = 0; c < NC; ++c)
 #pragma unroll
@@ -262,6 +277,20 @@ __device__ __forceinline__ void tile_part(const uint8_t *stage, int pitch, int w
   const float ng = __half2float(__ushort_as_half((unsigned short)(hg.x >> 16))) * 64.0f;
   const float dh = __half2float(__ushort_as_half((unsigned short)(hh.x & 0xffffu))) * 16777216.0f;
   const float nh = __half2float(__ushort_as_half((unsigned short)(hh.x >> 16))) * 64.0f;
+  if (PL == 1) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float sg = 0.f, sh = 0.f;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        sg += ce[0][c][i] + co[0][c][i];
+        sh += ce[0][c][2 + i] + co[0][c][2 + i];
+      }
+      rg[i] = dg * sg - ng * cm[0][i];
+      rh[i] = dh * sh - nh * cm[0][2 + i];
+    }
+    return;
+  }
 #pragma unroll
   for (int q = 0; q < NG; ++q) {
     float sg = 0.f, sh = 0.f;
@@ -296,8 +325,8 @@ struct PhaseSmem {       // per CTA
   uint8_t *ring;         // kWarps * stages * sbs * kStageBytes
   uint8_t *panels;       // kJobTok * nsb * kPanelBytes: the panels of the job in progress
   uint64_t *bars;        // kWarps * kMaxStages, initialised with count 1
-  float *inv;            // [kJobTok][16]
-  int *pair;             // [kJobTok]: output rows of the job's tokens, -1: no token in the slot
+  float *inv;            // [job_tokens][16]
+  int *pair;             // [job_tokens]: output rows of the job's tokens, -1: no token in the slot
   float4 *red;           // [kWarps][32]: partial sums of the warps that share a tile (ksplit > 1 only)
   volatile int *fail;    // raised by the first wait that gives up
 };
@@ -326,7 +355,7 @@ __device__ __forceinline__ int job_locate(const int *jbase, int job) {
 // ksplit (1, 2 or 4, a divisor of the boxes per tile): that many adjacent warps share a tile, each taking a
 // contiguous part of its K range; their partial sums meet in sm.red (fixed order, two named barriers per tile).
 // For runs with few tiles per warp, where a warp walking the whole K alone would be the critical path.
-template <bool DUAL, class JobToken, class LoadRow>
+template <bool DUAL, int PL = 2, class JobToken, class LoadRow>
 __device__ __forceinline__ void run_phase(const PhaseShape &sh, const PhaseSmem &sm, const JobTable &jt, int u0, int u1,
                                           int ksplit, const CUtensorMap *map0, const CUtensorMap *map1, float *out0,
                                           float *out1, float *out2, long long wait_cycles, unsigned &parity, bool &ok,
@@ -377,7 +406,7 @@ __device__ __forceinline__ void run_phase(const PhaseShape &sh, const PhaseSmem 
 
     __syncthreads();  // the previous job's tiles are done with the panels
     // ---- panels of the job: one warp per (token, superblock)
-    for (int item = warp; item < kJobTok * nsb; item += kWarps) {
+    for (int item = warp; item < job_tokens<PL>() * nsb; item += kWarps) {
       const int sb = item % nsb, tk = item / nsb;
       int pair = -1, row = 0;
       const bool live = job_token(job, a, tk, pair, row);
@@ -385,14 +414,14 @@ __device__ __forceinline__ void run_phase(const PhaseShape &sh, const PhaseSmem 
         float v[8];
         load_row(row, sb, lane, v);
         if (trace_mode != 3) {
-          const float inv = panel_convert(v, sm.panels + (size_t)tk * tok_stride + (size_t)sb * kPanelBytes, lane);
+          const float inv = panel_convert<PL>(v, sm.panels + (size_t)(PL == 1 ? tk >> 1 : tk) * tok_stride + (size_t)sb * kPanelBytes, lane, tk & 1);
           if (lane == 0) sm.inv[tk * 16 + sb] = inv;
         }
       }
       if (sb == 0 && lane == 0) sm.pair[tk] = live ? pair : -1;
     }
     __syncthreads();
-    const bool two = kJobTok > 4 && sm.pair[kJobTok > 4 ? 4 : 0] >= 0;  // tokens fill the slots from 0 up: a fifth token means a second group
+    const bool two = PL == 2 && kJobTok > 4 && sm.pair[kJobTok > 4 ? 4 : 0] >= 0;  // tokens fill the slots from 0 up: a fifth token means a second group
 
     int stage = 0;
     int n0 = (r0 + slot - job * tiles) * rows_per_tile;  // first output row of the tile in progress
@@ -400,7 +429,7 @@ __device__ __forceinline__ void run_phase(const PhaseShape &sh, const PhaseSmem 
     for (int ti = 0; ti < n_mine; ++ti, n0 += groups * rows_per_tile) {
       float rg[2] = {0.f, 0.f}, rh[2] = {0.f, 0.f};
       const uint8_t *pan = sm.panels + (size_t)sb_first * kPanelBytes;
-      const float *inv = sm.inv + t * 16 + sb_first;
+      const float *inv = sm.inv + (PL == 1 ? 2 * t : t) * 16 + sb_first;
       for (int bl = 0; bl < nb; ++bl) {
         if (ok && trace_mode != 2) {
           if (!mbar_wait_for(&bars[stage], (parity >> stage) & 1u, wait_cycles, sm.fail)) ok = false;
@@ -411,7 +440,14 @@ __device__ __forceinline__ void run_phase(const PhaseShape &sh, const PhaseSmem 
             const uint8_t *src = ring + (size_t)stage * stage_bytes;
             for (int k = 0; k < sbs; ++k, src += KNJ_Q4K_BYTES, pan += kPanelBytes, ++inv) {
               auto nothing = [] {};
-              if (two) {
+              if constexpr (PL == 1) {
+                float pg[2], ph[2];
+                tile_part<1, 1>(src, pitch, wrow, pan, tok_stride, lane, pg, ph, nothing);
+                rg[0] = fmaf(pg[0], inv[0], rg[0]);
+                rh[0] = fmaf(ph[0], inv[0], rh[0]);
+                rg[1] = fmaf(pg[1], inv[16], rg[1]);
+                rh[1] = fmaf(ph[1], inv[16], rh[1]);
+              } else if (two) {
                 float pg[2], ph[2];
                 tile_part<2>(src, pitch, wrow, pan, tok_stride, lane, pg, ph, nothing);
                 rg[0] = fmaf(pg[0], inv[0], rg[0]);
@@ -448,7 +484,7 @@ __device__ __forceinline__ void run_phase(const PhaseShape &sh, const PhaseSmem 
       if (mine && ok) {
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-          const int pair = (q == 0 || two) ? sm.pair[4 * q + t] : -1;
+          const int pair = PL == 1 ? sm.pair[2 * t + q] : (q == 0 || two) ? sm.pair[4 * q + t] : -1;
           if (pair >= 0) {
             if (DUAL) {
               const size_t o = (size_t)pair * sh.N + n0 + wrow;

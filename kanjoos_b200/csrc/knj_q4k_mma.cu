@@ -66,14 +66,16 @@ __host__ __device__ inline ProjSmem proj_smem(int nsb, int sbs, int stages) {
 __device__ int g_trace_mode = 0;
 #endif
 
-// IDENT: one matrix and rows 0..n_ident-1 (a dense product); the plan's arrays are not read.
-template <bool DUAL, bool IDENT>
+// IDENT: one matrix and rows 0..n_ident-1 (a dense product); the plan's arrays are not read. PL = 1: rows of a 16-bit type,
+// eight to a job (301 bf16 rows of a 2048 x 2048 matrix: 46.6 -> 31.1 us).
+template <bool DUAL, bool IDENT, int PL>
 __global__ void __launch_bounds__(kThreads, 1) q4k_proj_kernel(const __grid_constant__ ProjParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ int s_jbase[257];
   __shared__ int s_uexp[256], s_ucnt[256];
-  __shared__ float s_inv[q4e::kJobTok * 16];
-  __shared__ int s_pair[q4e::kJobTok];
+  constexpr int kTok = q4e::job_tokens<PL>();
+  __shared__ float s_inv[kTok * 16];
+  __shared__ int s_pair[kTok];
   __shared__ int s_fail;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const ProjSmem lay = proj_smem(p.shape.nsb, p.shape.sbs, p.shape.stages);
@@ -103,7 +105,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_proj_kernel(const __grid_cons
     }
     s_uexp[a] = ex;
     s_ucnt[a] = c;
-    s_jbase[a] = (c + q4e::kJobTok - 1) / q4e::kJobTok;
+    s_jbase[a] = (c + kTok - 1) / kTok;
   }
   __syncthreads();
   if (warp == 0) q4e::job_prefix(s_jbase, lane);
@@ -118,10 +120,10 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_proj_kernel(const __grid_cons
 #ifdef KNJ_TRACE
   tmode = g_trace_mode;
 #endif
-  q4e::run_phase<DUAL>(
+  q4e::run_phase<DUAL, PL>(
       p.shape, sm, jt, u0, u1, q4e::choose_ksplit(U, p.shape.nsb / p.shape.sbs, gridDim.x), &p.map0, &p.map1, p.out0, p.out1, p.out2, p.wait_cycles, parity, ok,
       [&](int job, int a, int tk, int &pair, int &row) {
-        const int tok = (job - s_jbase[a]) * q4e::kJobTok + tk;
+        const int tok = (job - s_jbase[a]) * kTok + tk;
         if (tok >= s_ucnt[a]) return false;
         pair = IDENT ? tok : p.pair_idx[(size_t)s_uexp[a] * p.idxStride + tok];
         row = p.row_map ? p.row_map[pair] : pair / p.row_div;
@@ -136,9 +138,9 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_proj_kernel(const __grid_cons
     __syncthreads();
     if (*sm.fail) {
       const int tiles = p.shape.tiles;
-      for (long long i = threadIdx.x; i < (long long)(u1 - u0) * q4e::kJobTok * 16; i += kThreads) {
-        const int u = u0 + (int)(i / (q4e::kJobTok * 16)), tk = (int)(i / 16) % q4e::kJobTok;
-        const int tok = u / tiles * q4e::kJobTok + tk;
+      for (long long i = threadIdx.x; i < (long long)(u1 - u0) * kTok * 16; i += kThreads) {
+        const int u = u0 + (int)(i / (kTok * 16)), tk = (int)(i / 16) % kTok;
+        const int tok = u / tiles * kTok + tk;
         if (tok < p.n_ident) p.out0[(size_t)tok * p.shape.N + u % tiles * 16 + (int)(i % 16)] = __int_as_float(0x7fffffff);
       }
     }
@@ -148,7 +150,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_proj_kernel(const __grid_cons
 long long g_decode_wait_cycles = kMaxWaitCycles;
 thread_local int t_stall_dense = 0;  // knj_q4k_matmul_test_stall
 
-template <bool DUAL, bool IDENT = false>
+template <bool DUAL, bool IDENT = false, int PL = 2>
 int launch_proj(ProjParams p, int n_experts_max, cudaStream_t st) {
   const int nsb = p.K / KNJ_QK_K;
   KNJ_REQUIRE(nsb >= 1 && nsb <= 16, "q4k projection: rows of %d weights (at most 4096 are taken)", p.K);
@@ -177,7 +179,7 @@ int launch_proj(ProjParams p, int n_experts_max, cudaStream_t st) {
   while (p.shape.stages > 2 && proj_smem(nsb, p.shape.sbs, p.shape.stages).total + reserve > (size_t)smem_max) --p.shape.stages;
   const size_t smem = proj_smem(nsb, p.shape.sbs, p.shape.stages).total;
   KNJ_REQUIRE(smem + reserve <= (size_t)smem_max, "q4k projection: rows of %d weights do not fit the shared memory", p.K);
-  auto kern = q4k_proj_kernel<DUAL, IDENT>;
+  auto kern = q4k_proj_kernel<DUAL, IDENT, PL>;
   // opt in to the large dynamic shared memory once per device and instantiation
   // (kept out of later launches so they are plain stream work, capturable in a graph)
   static size_t opted[64] = {0};
@@ -213,6 +215,13 @@ int dense_product(const uint8_t *W, int n_in, int n_out, const void *x, int x_dt
   p.W0 = W; p.X = x; p.x_dtype = x_dtype; p.ldx = ldx; p.n_ident = m;
   p.out0 = y; p.shape.N = n_out; p.K = n_in; p.row_div = 1;
   p.shape.tiles = n_out / 16; p.idxStride = m; p.stall = t_stall_dense;
+  // 16-bit rows hold in one plane of the panel (the other one would be all zeros), so twice as many can make a job: half the
+  // unpacking, but also half the jobs to spread over 2368 warps. bf16, us, jobs of four / of eight, with the tiles of the
+  // former and their superblocks in all: 16 x 768 x 2048 (192, 1.5 k) 7.4 / 8.1, 33 x 2048 x 1024 (1152, 4.6 k) 10.1 / 10.3,
+  // 9 x 4096 x 4096 (768, 12 k) 20.3 / 15.3, 512 x 256 x 256 (2048, 2 k) 7.5 / 7.0, 64 x 2048 x 2048 (2048, 16 k) 18.3 / 16.2,
+  // 512 x 4096 x 4096 229 / 132.
+  const long long tiles4 = (long long)((m + 3) / 4) * p.shape.tiles;
+  if (x_dtype != KNJ_DT_F32 && (tiles4 >= 2048 || tiles4 * (n_in / KNJ_QK_K) >= 8192)) return launch_proj<false, true, 1>(p, 1, as_stream(s));
   return launch_proj<false, true>(p, 1, as_stream(s));
 }
 

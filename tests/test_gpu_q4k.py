@@ -102,6 +102,23 @@ def test_matmul_16bit_activations(dtype):
     assert report(got, want, f"matmul {dtype}")["rel_rmse"] <= TOL_F32
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("m,n_in,n_out", [(7, 768, 48), (9, 4096, 4096), (65, 512, 2048), (301, 768, 432), (512, 256, 256)])
+def test_matmul_16bit_rows_in_jobs_of_eight(m, n_in, n_out, dtype):
+    """Enough 16-bit rows travel as one plane, eight to a job (the first case: too few, jobs of four): full and ragged jobs,
+    odd and even superblock counts, K split and not, rows over eight decades of magnitude (float16: subnormal ones
+    included), against a float64 product of the decode."""
+    from kanjoos_b200 import ops
+    rng = np.random.Generator(np.random.Philox([m, n_in, n_out]))
+    W = synth.q4k_rows(rng, n_out, n_in)
+    scale = 10.0 ** (rng.integers(-4, 4, size=(m, 1)) if dtype == torch.bfloat16 else rng.integers(-6, 2, size=(m, 1)))
+    x = torch.from_numpy((rng.standard_normal((m, n_in)) * scale).astype(np.float32)).to(dtype)
+    got = product_into(dev(W), x.cuda(), torch.full((m, n_out), SENTINEL, dtype=torch.float32, device="cuda")).cpu().numpy()
+    want = x.double().numpy() @ ol.dequant_q4k(W).reshape(n_out, n_in).astype(np.float64).T
+    err = np.sqrt(((got - want) ** 2).mean(1)) / np.sqrt((want ** 2).mean(1))
+    assert (got != SENTINEL).all() and err.max() <= 2e-6, f"row {err.argmax()}: {err.max():.2e}"   # f32 sums of n_in products
+
+
 def test_matmul_wide_dynamic_range():
     """Activations spanning 12 orders of magnitude, a zero row and tiny rows: the
     per-vector scaling of the activation planes must keep f32-level accuracy."""
