@@ -277,5 +277,109 @@ __device__ __forceinline__ bool chunk_pass(const Bufs &b, const uint8_t *src, in
   return true;
 }
 
+// ---- whole-tile form (the down phase of the whole-stack launch) ------------------------------------------------
+// A warp owns a tile of 16 rows for the whole K, as in the Q4_K engine: the tile's superblocks are contiguous
+// (3360 bytes a superblock column, a multiple of 16) and travel as one bulk copy into a buffer of the warp's own, so no
+// warp waits for another. The panel holds four tokens, two planes each, under a scale per (token, superblock).
+constexpr int kTileTok = 4;
+__host__ __device__ inline size_t tile_bytes(int nsb) { return (size_t)16 * nsb * KNJ_Q6K_BYTES; }
+__host__ __device__ inline size_t tile_panel_bytes(int nsb) { return (size_t)nsb * 16 * 32 * 8; }  // [16 k-steps][32 lanes] x 8 bytes
+
+// One warp converts the 256 values of (token slot tk, superblock sb), lane l holding values 8 l .. 8 l + 7, into the
+// B fragments of its sixteen k-steps; returns 1 / scale (the same in every lane).
+__device__ __forceinline__ float tile_panel_convert(const float (&v)[8], uint8_t *panel, int sb, int tk, int lane) {
+  float amax = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+  amax = warp_max(amax);
+  // power-of-two scale that puts the largest magnitude in [2^13, 2^14)
+  const int be = (int)(__float_as_uint(amax) >> 23);
+  int e = 0;
+  if (amax > 0.f && be != 0xff) e = max(-120, min(120, 140 - be));
+  const float s = __uint_as_float((uint32_t)(127 + e) << 23);
+  uint32_t hw[4], lw[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float f0 = v[2 * i] * s, f1 = v[2 * i + 1] * s;
+    const __half h0 = __float2half_rn(f0), h1 = __float2half_rn(f1);
+    const __half l0 = __float2half_rn(f0 - __half2float(h0)), l1 = __float2half_rn(f1 - __half2float(h1));
+    hw[i] = (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16);
+    lw[i] = (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16);
+  }
+  // lane (g, t) of a k-step holds activations 4 t .. 4 t + 3 of token g / 2, plane g % 2
+  uint8_t *at = panel + ((size_t)(16 * sb + (lane >> 1)) * 32 + 8 * tk + 2 * (lane & 1)) * 8;
+  *reinterpret_cast<uint4 *>(at) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+  *reinterpret_cast<uint4 *>(at + 32) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+  return __uint_as_float((uint32_t)(127 - e) << 23);
+}
+
+// A tile against the panel: lane (g, t) receives rows g and g + 8 for token t. inv: 1 / scale of that token's superblocks.
+// An int8 scale becomes a float as 2^23 + 128 + sc, less 2^23 + 128 (exact): the conversion instruction runs at a quarter
+// of the rate and was one per scale group and row.
+__device__ __forceinline__ void tile_mma(const uint8_t *wbuf, const uint8_t *panel, const float *inv, int nsb, int lane, float &y0, float &y1) {
+  const int g = lane >> 2, t = lane & 3, row_bytes = nsb * KNJ_Q6K_BYTES;
+  const __half2 k1056 = __float2half2_rn(1056.0f);  // 1024 (the byte-to-fp16 trick) + 32 (the code's offset)
+  const uint8_t *r[2] = {wbuf + (size_t)g * row_bytes, wbuf + (size_t)(g + 8) * row_bytes};
+  const uint2 *bp = reinterpret_cast<const uint2 *>(panel) + lane;
+  y0 = y1 = 0.f;
+#pragma unroll 1
+  for (int sb = 0; sb < nsb; ++sb) {
+    // rows are 2-byte aligned: a word is put together from two aligned ones, all words of a superblock alike
+    const uint32_t *w[2];
+    uint32_t sel[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uintptr_t a = reinterpret_cast<uintptr_t>(r[i] + sb * KNJ_Q6K_BYTES);
+      w[i] = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
+      sel[i] = (a & 2) ? 0x5432u : 0x3210u;
+    }
+    auto word = [&](int i, int byte) { return __byte_perm(w[i][byte >> 2], w[i][(byte >> 2) + 1], sel[i]); };
+    float p0 = 0.f, p1 = 0.f;
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      uint32_t sc[2][2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) sc[i][q] = word(i, 192 + 8 * hf + 4 * q) ^ 0x80808080u;
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {
+        const int off = 16 * hh + 4 * t;
+        uint32_t qh[2], ql[2][2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          qh[i] = word(i, 128 + 32 * hf + off);
+          ql[i][0] = word(i, 64 * hf + off);
+          ql[i][1] = word(i, 64 * hf + 32 + off);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          __half2 a[2][2];
+          float s[2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const uint32_t nib = (c & 2 ? ql[i][c & 1] >> 4 : ql[i][c & 1]) & 0x0f0f0f0fu;
+            const uint32_t q = nib | ((c < 2 ? qh[i] << (4 - 2 * c) : qh[i] >> (2 * c - 4)) & 0x30303030u);
+            const uint32_t e0 = __byte_perm(q, 0x64646464u, 0x4140), e1 = __byte_perm(q, 0x64646464u, 0x4342);
+            a[i][0] = __hsub2(*reinterpret_cast<const __half2 *>(&e0), k1056);
+            a[i][1] = __hsub2(*reinterpret_cast<const __half2 *>(&e1), k1056);
+            s[i] = __uint_as_float(__byte_perm(sc[i][c >> 1], 0x4b000000u, 0x7650u | (uint32_t)(2 * (c & 1) + hh))) - 8388736.0f;
+          }
+          const uint2 bf = bp[(size_t)(16 * sb + 8 * hf + 2 * c + hh) * 32];
+          float m[4];
+          mma_f16_16816_zero(m, *reinterpret_cast<const uint32_t *>(&a[0][0]), *reinterpret_cast<const uint32_t *>(&a[1][0]),
+                             *reinterpret_cast<const uint32_t *>(&a[0][1]), *reinterpret_cast<const uint32_t *>(&a[1][1]), bf.x, bf.y);
+          p0 = fmaf(s[0], m[0] + m[1], p0);
+          p1 = fmaf(s[1], m[2] + m[3], p1);
+        }
+      }
+    }
+    const float d0 = knj_half_bits_to_float(*reinterpret_cast<const uint16_t *>(r[0] + sb * KNJ_Q6K_BYTES + 208));
+    const float d1 = knj_half_bits_to_float(*reinterpret_cast<const uint16_t *>(r[1] + sb * KNJ_Q6K_BYTES + 208));
+    y0 = fmaf(d0 * p0, inv[sb], y0);
+    y1 = fmaf(d1 * p1, inv[sb], y1);
+  }
+}
+
 }  // namespace q6b
 }  // namespace knj

@@ -125,7 +125,7 @@ __host__ __device__ inline Plan make_plan(const q4e::PhaseShape &gu, const q4e::
   pl.pair = take(q4e::kJobTok * 4);
   pl.scale = take((size_t)T * 4);
   pl.ord = take((size_t)T * k);
-  pl.fail = take(32);   // fail word, then the two block barriers of the Q6_K down phase
+  pl.fail = take(32);
   pl.desc = take(2 * sizeof(LayerDesc));
   // partial sums of warps that share a tile: only small batches have so few tiles that they do
   pl.red = T <= kSplitMaxT ? take((size_t)q4e::kWarps * 32 * sizeof(float4)) : 0;
@@ -350,54 +350,76 @@ __device__ __noinline__ void stage_plan(const StackParams &p, const LayerDesc &L
 
 }
 
-// Down phase of a layer whose down matrices are Q6_K: (active expert, one to four blocks of 64 output rows) units
-// dealt round robin over the CTAs; the blocks' superblocks and the activation side of up to eight of the expert's
-// tokens live in the (idle) ring area, the arithmetic is knj_q6k_block.cuh's, i.e. the stand-alone projection's.
-// Where the blocks can travel as bulk copies (16-byte aligned base, H a multiple of 64) and the ring area holds two
-// of them, the next block is under way while this one is worked on: two barriers behind the fail word, `staged`
-// counts this CTA's blocks over the whole launch.
-__device__ __noinline__ void stage_down_q6k(const StackParams &p, const LayerDesc &L, const Plan &pl, uint8_t *smem, unsigned &staged,
+// Down phase of a layer whose down matrices are Q6_K: the CTA's run of the flat (job, 16-row tile) list, as in the Q4_K
+// engine, with q6b's whole tiles: a warp copies a tile of its own (10 KB at ffn 768), multiplies it and asks for the next.
+// The buffers lie in the ring area and the panel behind them; where sixteen do not fit (ffn 1024) fewer warps take tiles.
+// Before, blocks of 64 rows were staged and reduced by the whole CTA, three CTA barriers each: 45 us on the mean and 60 to
+// the last CTA at 8 tokens (51 experts, 66 MB, 10 us of HBM time), where the Q4_K phase takes 18.
+__device__ __noinline__ void stage_down_q6k(const StackParams &p, const LayerDesc &L, const Plan &pl, uint8_t *smem, unsigned &parity,
                                             bool &ok) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int H = p.H, F = p.F, k = p.k, c = blockIdx.x, G = gridDim.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int H = p.H, F = p.F, k = p.k, c = blockIdx.x, G = gridDim.x, tiles = p.dn.tiles, nsb = p.dn.nsb;
   const int *sel_e = reinterpret_cast<const int *>(smem + pl.sel_e);
   const unsigned long long *mask = reinterpret_cast<const unsigned long long *>(smem + pl.mask);
   const int *jbase = reinterpret_cast<const int *>(smem + pl.jbase), *uexp = reinterpret_cast<const int *>(smem + pl.uexp);
-  int *s_pair = reinterpret_cast<int *>(smem + pl.inv);  // eight ints: the pass's output rows (the phase engine is idle)
-  const int row_bytes = F / KNJ_QK_K * KNJ_Q6K_BYTES;
-  const bool two = 2 * q6b::block_bytes(F) + q6b::act_scratch_bytes(F, q4e::kWarps) <= (size_t)(pl.panels - pl.ring);
-  const bool bulk = (reinterpret_cast<uintptr_t>(L.w_down6) & 15u) == 0 && H % q6b::kRows == 0;
-  const q6b::Bufs b = q6b::carve(smem + pl.ring, F, q4e::kWarps, two, reinterpret_cast<uint64_t *>(smem + pl.fail + 16),
-                                 reinterpret_cast<int *>(smem + pl.fail));
-  const int blocks = (H + q6b::kRows - 1) / q6b::kRows, n_act = jbase[259];
-  const int sub = max(1, min(4, n_act * blocks / (2 * G)));  // blocks per unit: the activation side is prepared once per unit
-  const int chunks = (blocks + sub - 1) / sub, total = n_act * chunks;
-  for (int u = c; u < total; u += G) {
-    const int a = u / chunks, ch = u - a * chunks;
-    const int e = uexp[a];
-    const int n0 = ch * sub * q6b::kRows, n_rows = min(sub * q6b::kRows, H - n0);
-    unsigned long long m = mask[e];
-    while (m) {
-      __syncthreads();  // the previous pass is done with the shared buffers
-      // the pass's tokens are the lowest set bits of the mask: thread 8 i + j looks at slot j (+ 8, ...) of the i-th
-      const int nt = min(q6b::kTok, __popcll(m));
-      if (threadIdx.x < 8 * q6b::kTok) {
-        const int i = threadIdx.x >> 3;
-        unsigned long long mm = m;
-        for (int x = 0; x < i; ++x) mm &= mm - 1;
-        if (i < nt) {
-          const int tok = __ffsll((long long)mm) - 1;
-          for (int j = threadIdx.x & 7; j < k; j += 8)
-            if (sel_e[tok * k + j] == e) s_pair[i] = tok * k + j;
-        }
+  float *inv = reinterpret_cast<float *>(smem + pl.inv);
+  int *s_pair = reinterpret_cast<int *>(smem + pl.pair);
+  volatile int *fail = reinterpret_cast<volatile int *>(smem + pl.fail);
+  const uint32_t tb = (uint32_t)q6b::tile_bytes(nsb);
+  const int nw = min(q4e::kWarps, (int)((pl.bars - pl.ring - (uint32_t)q6b::tile_panel_bytes(nsb)) / tb));
+  uint8_t *buf = smem + pl.ring + (size_t)warp * tb, *panel = smem + pl.ring + (size_t)nw * tb;
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem + pl.bars) + warp * q4e::kMaxStages;
+  static_assert(q6b::kTileTok == q4e::kJobTok, "one job table");
+  const long long U = (long long)jbase[256] * tiles;
+  const int u0 = (int)(U * c / G), u1 = (int)(U * (c + 1) / G);
+  if (u0 >= u1) return;
+  for (int job = u0 / tiles; job <= (u1 - 1) / tiles; ++job) {
+    const int a = q4e::job_locate(jbase, job), e = uexp[a];
+    const int r0 = max(u0, job * tiles), r1 = min(u1, (job + 1) * tiles);
+    const uint8_t *src = L.w_down6 + ((size_t)e * H - (size_t)job * tiles * 16) * (tb / 16);
+    auto issue = [&](int tile) {
+      if (lane == 0) {
+        fence_proxy_async();  // the buffer was read through the generic proxy
+        mbar_expect_tx(bar, tb);
+        bulk_g2s(buf, src + (size_t)tile * tb, tb, bar);
       }
-      for (int i = 0; i < nt; ++i) m &= m - 1;
-      __syncthreads();
-      if (!q6b::chunk_pass<q4e::kWarps>(b, L.w_down6 + ((size_t)e * H + n0) * row_bytes, n_rows, F, p.act, p.Y + n0, H, s_pair, nt, staged,
-                                        bulk, p.wait_cycles, lane, warp)) {
-        ok = false;  // a copy that never completes: bounded wait, the launch reports it
-        m = 0;
-        u = total;
+    };
+    int tile = warp < nw ? r0 + warp : r1;
+    if (ok && tile < r1) issue(tile);
+    __syncthreads();  // the previous job's tiles are done with the panel
+    // ---- the job's tokens: the (4 (job - first job of the expert))-th and following of the expert's set
+    for (int item = warp; item < q4e::kJobTok * nsb; item += q4e::kWarps) {
+      const int sb = item % nsb, tk = item / nsb, idx = (job - jbase[a]) * q4e::kJobTok + tk;
+      unsigned long long m = mask[e];
+      int pair = -1;
+      if (idx < __popcll(m)) {
+        for (int i = 0; i < idx; ++i) m &= m - 1ull;
+        const int tok = __ffsll((long long)m) - 1;
+        for (int j = 0; j < k; ++j) pair = sel_e[tok * k + j] == e ? tok * k + j : pair;
+        float v[8];
+        q4e::load8_f32(p.act, KNJ_DT_F32, (int64_t)pair * F + 256 * sb + 8 * lane, v);
+        const float iv = q6b::tile_panel_convert(v, panel, sb, tk, lane);
+        if (lane == 0) inv[tk * 16 + sb] = iv;
+      }
+      if (sb == 0 && lane == 0) s_pair[tk] = pair;
+    }
+    __syncthreads();
+    for (; tile < r1; tile += nw) {
+      if (ok) {
+        if (!mbar_wait_for(bar, parity & 1u, p.wait_cycles, fail)) ok = false;
+        parity ^= 1u;
+      }
+      if (ok) {
+        float y0, y1;
+        q6b::tile_mma(buf, panel, inv + t * 16, nsb, lane, y0, y1);
+        __syncwarp();  // every lane is done with the buffer
+        if (tile + nw < r1) issue(tile + nw);
+        const int pair = s_pair[t];
+        if (pair >= 0) {
+          float *y = p.Y + (size_t)pair * H + (tile - job * tiles) * 16 + g;
+          y[0] = y0;
+          y[8] = y1;
+        }
       }
     }
   }
@@ -431,16 +453,12 @@ __global__ void __launch_bounds__(kThreads, 1) moe_stack_kernel(const StackParam
     for (int s = 0; s < q4e::kMaxStages; ++s) mbar_init(&sm.bars[warp * q4e::kMaxStages + s], 1);
   if (threadIdx.x == 0) {
     *s_fail = 0;
-    // the Q6_K down phase's two block barriers (behind the fail word)
-    mbar_init(reinterpret_cast<uint64_t *>(smem + pl.fail + 16), 1);
-    mbar_init(reinterpret_cast<uint64_t *>(smem + pl.fail + 24), 1);
   }
   mbar_init_fence();
   __syncthreads();
 
   unsigned arrivals = 0, parity = 0;
   bool ok = true;
-  unsigned q6_staged = 0;  // Q6_K down blocks this CTA has staged so far (stage_down_q6k)
   // logits: CTA c < n_eg * n_tg takes experts epi * eg .. + epi - 1 for tokens 8 tg .. 8 tg + 7
   const int n_tg = (T + 7) / 8;
   int epi = 8;
@@ -531,7 +549,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_stack_kernel(const StackParam
     KNJ_STAMP(5);
 
     // ---- stage 4: down -> Y (one row per pair)
-    if (L.w_down6) stage_down_q6k(p, L, pl, smem, q6_staged, ok);
+    if (L.w_down6) stage_down_q6k(p, L, pl, smem, parity, ok);
     else {
       const long long U = (long long)jbase[256] * p.dn.tiles;
       const int u0 = (int)(U * c / G), u1 = (int)(U * (c + 1) / G);

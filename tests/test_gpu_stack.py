@@ -132,6 +132,24 @@ def test_mixed_format_stack_q6k_down_follows_the_layer_launches(T):
     st.close()
 
 
+@pytest.mark.parametrize("F,T", [(256, 1), (256, 20), (768, 5), (768, 33), (1024, 3), (1024, 20)])
+def test_q6k_down_phase_follows_the_layer_launch_at_every_row_length(F, T):
+    """One Q6_K layer: tiles of one, three and four superblocks (four leave room for twelve warps' tiles, not sixteen),
+    experts of one and of several jobs of four tokens, against the layer launch's own Q6_K projection."""
+    from kanjoos_b200.moe import ExpertBank, FusedMoeStack, MoeFfnLayer
+    E, H, k = 12, 512, 4
+    bank = dict(synth.expert_bank(808, 0, n_experts=E, hidden=H, ffn=F), down=_q6k_down(808, E, H, F))
+    wr, _ = synth.router_weight(808, 0, n_experts=E, hidden=H)
+    b = ExpertBank.from_numpy(bank, wr, None, synth.norm_weight(808, 0, H))
+    x = dev(synth.hidden_rows(808, T, H))
+    want = MoeFfnLayer(b, top_k=k, max_tokens=T, residual=True).decode(x).cpu().numpy()
+    st = FusedMoeStack([b], top_k=k, n_tokens=T, dtype=torch.float32)
+    got = st.step(x).cpu().numpy()
+    st.status()
+    st.close()
+    assert report(got, want, f"Q6_K down phase, ffn {F}, T={T}")["rel_rmse"] <= 1e-5
+
+
 @pytest.mark.parametrize("B", [1, 8, 64])
 def test_config4_full_size_stack_checked_layers(B):
     """Config 4: the 48-layer resident stack at full size (about 15 GiB of random-init Q4_K experts), f32 residual
