@@ -286,7 +286,7 @@ __device__ __noinline__ void stage_plan(const StackParams &p, const LayerDesc &L
         int e[kNt];
 #pragma unroll
         for (int n = 0; n < kNt; ++n) topk_load<kEpl>(p.logits + (size_t)min(t0 + q4e::kWarps * n, T - 1) * E, E, lane, v[n]);
-        warp_topk<kEpl, kNt>(v, k, lane, e, w);
+        warp_topk<kEpl, kNt>(v, E, k, lane, e, w);
 #pragma unroll
         for (int n = 0; n < kNt; ++n) {
           const int t = t0 + q4e::kWarps * n;

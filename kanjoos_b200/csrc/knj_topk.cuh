@@ -8,7 +8,11 @@ namespace knj {
 // ---------------------------------------------------------------------------
 // Softmax + exact top-k + renormalise: one warp per token. Selection is by
 // (value descending, expert id ascending), the tie rule of the CPU path's
-// strict '>' scan (src/model/model.cpp:442-451).
+// strict '>' scan (src/model/model.cpp:442-451). An expert with logit -inf
+// (masked by its bias) is a candidate like any other, below every finite one:
+// with fewer than k finite logits the rest are the masked experts of lowest id,
+// weight 0, as in the CPU path, so that a selection is always an expert of the
+// layer (it indexes tables). A row of -inf alone has weights 0.
 // ---------------------------------------------------------------------------
 constexpr int kMaxEPerLane = 8;  // E <= 256
 
@@ -20,14 +24,14 @@ __device__ __forceinline__ void topk_load(const float *lg, int E, int lane, floa
 }
 
 // One warp: softmax over the E logits of a token (topk_load), exact top-k, renormalised weights. Lane s < k ends up with
-// the s-th selection. E <= 32 * EPL; fewer experts per lane than the maximum only shortens the loops.
+// the s-th selection. k <= E <= 32 * EPL; fewer experts per lane than the maximum only shortens the loops.
 // A token's selection is one dependent chain, so it is kept short: every lane sorts its own few keys first (stable, so
 // equal keys stay in id order), and a round is then one warp maximum over the lanes' heads, one ballot, and the
 // winner's queue moving up; the values are fetched from the winner off the chain, and only the k selected are divided by
 // the softmax sum. (Two warp reductions, a scan and a shuffle in each round, and EPL divisions, took 2.2 us a token.)
 // NT tokens at a time share the chain's latency: their steps are independent of each other.
 template <int EPL, int NT>
-__device__ __forceinline__ void warp_topk(const float (&v)[NT][EPL], int k, int lane, int (&sel_e)[NT], float (&sel_w)[NT]) {
+__device__ __forceinline__ void warp_topk(const float (&v)[NT][EPL], int E, int k, int lane, int (&sel_e)[NT], float (&sel_w)[NT]) {
   float mx[NT], sum[NT], ex[NT][EPL];
   unsigned key[NT][EPL];
   int id[NT][EPL];
@@ -44,13 +48,13 @@ __device__ __forceinline__ void warp_topk(const float (&v)[NT][EPL], int k, int 
 #pragma unroll
   for (int n = 0; n < NT; ++n) {
     sum[n] = 0.f;
-    sel_e[n] = 0x7fffffff;
+    sel_e[n] = 0;
     sel_w[n] = 0.f;
 #pragma unroll
     for (int i = 0; i < EPL; ++i) {
-      // order-preserving integer keys: larger float <=> larger unsigned key; 0 for none
+      // order-preserving integer keys: larger float <=> larger unsigned key; 0 only past the last expert
       const unsigned u = __float_as_uint(v[n][i]);
-      key[n][i] = (v[n][i] == -INFINITY) ? 0u : ((u & 0x80000000u) ? ~u : (u | 0x80000000u));
+      key[n][i] = i * 32 + lane < E ? max(1u, (u & 0x80000000u) ? ~u : (u | 0x80000000u)) : 0u;
       ex[n][i] = (v[n][i] == -INFINITY) ? 0.f : expf(v[n][i] - mx[n]);
       sum[n] += ex[n][i];
       id[n][i] = i * 32 + lane;
@@ -77,16 +81,16 @@ __device__ __forceinline__ void warp_topk(const float (&v)[NT][EPL], int k, int 
     for (int n = 0; n < NT; ++n) top[n] = __reduce_max_sync(0xffffffffu, key[n][0]);
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
-      const unsigned holders = __ballot_sync(0xffffffffu, key[n][0] == top[n] && top[n] != 0u);
+      const unsigned holders = __ballot_sync(0xffffffffu, key[n][0] == top[n]);
       src[n] = __ffs(holders) - 1;
       if (holders & (holders - 1u))  // equal logits: the smallest id among the lanes that hold one
         src[n] = __reduce_min_sync(0xffffffffu, key[n][0] == top[n] ? id[n][0] : 0x7fffffff) & 31;
     }
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
-      const int e = __shfl_sync(0xffffffffu, id[n][0], src[n] & 31);
-      const float x = __shfl_sync(0xffffffffu, ex[n][0], src[n] & 31);
-      if (lane == s && src[n] >= 0) {  // none left: fewer than k candidates
+      const int e = __shfl_sync(0xffffffffu, id[n][0], src[n]);
+      const float x = __shfl_sync(0xffffffffu, ex[n][0], src[n]);
+      if (lane == s) {
         sel_e[n] = e;
         sel_w[n] = x;
       }
@@ -104,7 +108,7 @@ __device__ __forceinline__ void warp_topk(const float (&v)[NT][EPL], int k, int 
   float keep[NT];
 #pragma unroll
   for (int n = 0; n < NT; ++n) {
-    sel_w[n] = sel_w[n] / sum[n];
+    sel_w[n] = sum[n] == 0.f ? 0.f : sel_w[n] / sum[n];  // no finite logit: 0, not 0 / 0
     keep[n] = 0.f;
   }
 #pragma unroll
@@ -125,11 +129,11 @@ __device__ __forceinline__ void warp_topk(const float *lg, int E, int k, int lan
   if (E <= 128) {
     float v[1][4];
     topk_load<4>(lg, E, lane, v[0]);
-    warp_topk<4, 1>(v, k, lane, e, w);
+    warp_topk<4, 1>(v, E, k, lane, e, w);
   } else {
     float v[1][kMaxEPerLane];
     topk_load<kMaxEPerLane>(lg, E, lane, v[0]);
-    warp_topk<kMaxEPerLane, 1>(v, k, lane, e, w);
+    warp_topk<kMaxEPerLane, 1>(v, E, k, lane, e, w);
   }
   sel_e = e[0];
   sel_w = w[0];

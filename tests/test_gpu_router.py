@@ -129,3 +129,24 @@ def test_topk_of_equal_logits(E):
         assert (pe.view(T, k).cpu().numpy() == want[None]).all(), case
         w = np.exp(bias[want].astype(np.float64))
         assert np.abs(pw.view(T, k).cpu().numpy() - (w / w.sum())[None]).max() < 1e-6
+
+
+@pytest.mark.parametrize("T", [3, 40])
+@pytest.mark.parametrize("E", [8, 128, 200])
+def test_topk_with_masked_experts(E, T):
+    """A bias of -inf masks an expert. With fewer than k finite logits the masked experts of lowest id follow the finite ones
+    with weight 0, in a row of -inf alone every weight is 0: never an id outside the layer, never NaN. Zero rows, so the
+    logits are the biases (the weights carry one expf and two divisions: 1e-6)."""
+    from kanjoos_b200 import ops
+    k, H = 8, 256
+    for finite in ([], [E - 1], [3, E - 2, 5], list(range(k))):
+        bias = np.full(E, -np.inf, np.float32)
+        bias[finite] = -0.25 * np.arange(len(finite))
+        _, pe, pw = ops.router_topk(torch.zeros((T, H), device="cuda"), torch.zeros((E, H), dtype=torch.bfloat16, device="cuda"), k, dev(bias))
+        masked = [e for e in range(E) if e not in finite]
+        assert (pe.view(T, k).cpu().numpy() == (finite + masked)[:k]).all(), finite
+        w = np.zeros(k)
+        if finite:
+            w[:len(finite)] = np.exp(bias[finite].astype(np.float64))
+            w /= w.sum()
+        assert np.abs(pw.view(T, k).cpu().numpy() - w).max() < 1e-6, finite

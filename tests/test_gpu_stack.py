@@ -61,6 +61,29 @@ def test_routing_is_the_layer_launch_s_at_every_group_of_tokens(T, E):
     st.close()
 
 
+@pytest.mark.parametrize("T", [1, 2, 9, 33])
+def test_masked_experts(T):
+    """Biases of -inf that leave three experts to a top-4: the fourth is a masked one with weight 0, so the layer launch and
+    the stack (both kernels) give what top-3 gives, bit for bit; with every expert masked the rows pass through."""
+    from kanjoos_b200.moe import FusedMoeStack, MoeFfnLayer
+    E, H, F = 16, 512, 256
+    banks, _ = _banks(811, 1, E, H, F)
+    x = dev(synth.hidden_rows(811, T, H))
+    for finite in ([2, 7, 15], []):
+        bias = torch.full((E,), float("-inf"), device="cuda")
+        bias[finite] = 0.0
+        banks[0].router_bias = bias
+        want = MoeFfnLayer(banks[0], top_k=3, max_tokens=T, residual=True).decode(x) if finite else x
+        assert torch.equal(MoeFfnLayer(banks[0], top_k=4, max_tokens=T, residual=True).decode(x), want)
+        stacks = [FusedMoeStack(banks, top_k=k, n_tokens=T, dtype=torch.float32, taps=True) for k in (3, 4)]
+        got = [st.step(x).clone() for st in stacks]
+        for st in stacks:
+            st.status()
+            assert ((st.taps[0][0] >= 0) & (st.taps[0][0] < E)).all()
+            st.close()
+        assert torch.equal(got[1], got[0] if finite else x)
+
+
 def test_stack_follows_layer_by_layer_launches():
     from kanjoos_b200.moe import FusedMoeStack, MoeStack
     L, E, H, F, k, T = 6, 32, 1024, 512, 8, 2
