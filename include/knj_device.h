@@ -458,6 +458,11 @@ int knj_moe_stack_status(knj_moe_stack *st, knj_stream_t s);
  * and status() reports KNJ_E_TIMEOUT; 0 restores normal operation. Nothing traps
  * and the context stays usable. */
 int knj_moe_stack_set_wait(knj_moe_stack *st, long long wait_cycles, int stall_first_barrier);
+/* For tests as well: the first weight copies of warp 0..15 of one CTA never count
+ * as landed, from the next launch on, so the wait for them runs out as above;
+ * -1 restores normal operation. Refused for the stacks of one and two tokens
+ * (the scalar kernel waits for no such copy). */
+int knj_moe_stack_test_stall_copy(knj_moe_stack *st, int warp);
 void knj_moe_stack_destroy(knj_moe_stack *st);
 
 /* ======================================================================== */

@@ -108,6 +108,7 @@ SIGNATURES = {
     "knj_moe_stack_decode_launch": (_i, [_vp, _vp]),
     "knj_moe_stack_status": (_i, [_vp, _vp]),
     "knj_moe_stack_set_wait": (_i, [_vp, C.c_longlong, _i]),
+    "knj_moe_stack_test_stall_copy": (_i, [_vp, _i]),
     "knj_moe_stack_destroy": (None, [_vp]),
     "knj_res_arena_create": (_vp, []),
     "knj_res_arena_alloc": (_vp, [_vp, _u64]),

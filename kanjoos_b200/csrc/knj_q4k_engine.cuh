@@ -350,8 +350,9 @@ __device__ __forceinline__ int job_locate(const int *jbase, int job) {
 // exists and names its output row (pair) and its activation row; load_row(row, sb, lane, v) fetches values
 // 256 sb + 8 lane .. + 7 of that activation row. out0/out1/out2 as for the launches: DUAL -> G, U, silu(G) * U;
 // otherwise out0 = Y. Bit s of `parity` is the phase the warp's next wait on its barrier s expects (0 after
-// initialisation); `ok` turns false when a wait gave up (the rest of the phase is then skipped, the CTA barriers
-// are still met).
+// initialisation); `ok` turns false when a wait of this warp gave up (the rest of the phase is then skipped, the CTA
+// barriers are still met). Other warps may have landed all their boxes: what a CTA reports is *sm.fail, read behind a
+// CTA barrier, not one warp's `ok`.
 // ksplit (1, 2 or 4, a divisor of the boxes per tile): that many adjacent warps share a tile, each taking a
 // contiguous part of its K range; their partial sums meet in sm.red (fixed order, two named barriers per tile).
 // For runs with few tiles per warp, where a warp walking the whole K alone would be the critical path.
@@ -431,12 +432,13 @@ __device__ __forceinline__ void run_phase(const PhaseShape &sh, const PhaseSmem 
       const uint8_t *pan = sm.panels + (size_t)sb_first * kPanelBytes;
       const float *inv = sm.inv + (PL == 1 ? 2 * t : t) * 16 + sb_first;
       for (int bl = 0; bl < nb; ++bl) {
-        if (ok && trace_mode != 2) {
-          if (!mbar_wait_for(&bars[stage], (parity >> stage) & 1u, wait_cycles, sm.fail)) ok = false;
-          parity ^= 1u << stage;
-        }
         if (ok) {
-          if (trace_mode != 1) {
+          bool landed = true;
+          if (trace_mode != 2) {
+            landed = mbar_wait_warp(&bars[stage], (parity >> stage) & 1u, wait_cycles, sm.fail);
+            parity ^= 1u << stage;
+          }
+          if (trace_mode != 1) {  // not asked about `landed` yet (the vote's latency): sums of a box that did not land go nowhere
             const uint8_t *src = ring + (size_t)stage * stage_bytes;
             for (int k = 0; k < sbs; ++k, src += KNJ_Q4K_BYTES, pan += kPanelBytes, ++inv) {
               auto nothing = [] {};
@@ -463,7 +465,8 @@ __device__ __forceinline__ void run_phase(const PhaseShape &sh, const PhaseSmem 
             }
           }
           __syncwarp();  // every lane is done with the box
-          if (trace_mode != 2 && p_left > 0) issue_next();
+          ok = landed;
+          if (ok && trace_mode != 2 && p_left > 0) issue_next();
         }
         if (++stage == S) stage = 0;
       }

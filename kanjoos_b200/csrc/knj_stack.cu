@@ -20,7 +20,9 @@
 //
 // Every wait is bounded: a barrier or a copy that does not complete within the
 // limit sets the error word, every CTA that sees it returns, and
-// knj_moe_stack_status reports KNJ_E_TIMEOUT.
+// knj_moe_stack_status reports KNJ_E_TIMEOUT. A copy is waited for by one warp,
+// which raises the CTA's fail word; the next grid barrier turns that into the
+// error word, whichever warp it was.
 #include "knj_common.cuh"
 #include "knj_q4k.h"
 #include "knj_q4k_engine.cuh"
@@ -70,6 +72,7 @@ struct StackParams {
   q4e::PhaseShape gu, dn;
   long long wait_cycles;  // limit of every wait inside the kernel
   int stall;              // test hook: added to the first barrier's target, which then cannot complete
+  int stall_copy;         // test hook: w + 1 = the first copies of CTA 0's warp w never count as landed
 };
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
@@ -83,17 +86,22 @@ __device__ __forceinline__ void red_release(unsigned *p, unsigned v) {
 
 // Grid barrier in two halves, so that work that does not depend on the other CTAs can sit between them.
 // arrive: everything this CTA wrote so far is published. wait: all CTAs of the grid have arrived `target`
-// times in total; false: a wait ran out (here or elsewhere).
+// times in total; false: a wait ran out, this one, one elsewhere in the grid, or that for a copy of any warp of this
+// CTA (*fail, ordered by the CTA barrier of grid_arrive).
 __device__ __forceinline__ void grid_arrive(unsigned *sync) {
   __syncthreads();
   if (threadIdx.x == 0) red_release(sync, 1u);  // cumulative: releases what the CTA barrier ordered before it
 }
-__device__ __forceinline__ bool grid_wait(unsigned *sync, unsigned target, long long limit) {
+__device__ __forceinline__ bool grid_wait(unsigned *sync, volatile const int *fail, unsigned target, long long limit) {
   int ok = 1;
   if (threadIdx.x == 0) {
     const long long t0 = clock64();
     unsigned polls = 0;
-    while (ld_acquire(sync) < target) {
+    if (*fail) {
+      atomicExch(sync + 1, 1u);
+      ok = 0;
+    }
+    while (ok && ld_acquire(sync) < target) {
       if ((++polls & 63u) == 0u) {
         if (ld_acquire(sync + 1) != 0u) { ok = 0; break; }
         if (clock64() - t0 > limit) { atomicExch(sync + 1, 1u); ok = 0; break; }
@@ -355,8 +363,8 @@ __device__ __noinline__ void stage_plan(const StackParams &p, const LayerDesc &L
 // The buffers lie in the ring area and the panel behind them; where sixteen do not fit (ffn 1024) fewer warps take tiles.
 // Before, blocks of 64 rows were staged and reduced by the whole CTA, three CTA barriers each: 45 us on the mean and 60 to
 // the last CTA at 8 tokens (51 experts, 66 MB, 10 us of HBM time), where the Q4_K phase takes 18.
-__device__ __noinline__ void stage_down_q6k(const StackParams &p, const LayerDesc &L, const Plan &pl, uint8_t *smem, unsigned &parity,
-                                            bool &ok) {
+__device__ __noinline__ void stage_down_q6k(const StackParams &p, const LayerDesc &L, const Plan &pl, uint8_t *smem, unsigned &parity_io,
+                                            bool &ok_io) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int H = p.H, F = p.F, k = p.k, c = blockIdx.x, G = gridDim.x, tiles = p.dn.tiles, nsb = p.dn.nsb;
   const int *sel_e = reinterpret_cast<const int *>(smem + pl.sel_e);
@@ -373,6 +381,8 @@ __device__ __noinline__ void stage_down_q6k(const StackParams &p, const LayerDes
   const long long U = (long long)jbase[256] * tiles;
   const int u0 = (int)(U * c / G), u1 = (int)(U * (c + 1) / G);
   if (u0 >= u1) return;
+  unsigned parity = parity_io;
+  bool ok = ok_io;
   for (int job = u0 / tiles; job <= (u1 - 1) / tiles; ++job) {
     const int a = q4e::job_locate(jbase, job), e = uexp[a];
     const int r0 = max(u0, job * tiles), r1 = min(u1, (job + 1) * tiles);
@@ -406,16 +416,15 @@ __device__ __noinline__ void stage_down_q6k(const StackParams &p, const LayerDes
     __syncthreads();
     for (; tile < r1; tile += nw) {
       if (ok) {
-        if (!mbar_wait_for(bar, parity & 1u, p.wait_cycles, fail)) ok = false;
+        const bool landed = mbar_wait_warp(bar, parity & 1u, p.wait_cycles, fail);
         parity ^= 1u;
-      }
-      if (ok) {
         float y0, y1;
-        q6b::tile_mma(buf, panel, inv + t * 16, nsb, lane, y0, y1);
+        q6b::tile_mma(buf, panel, inv + t * 16, nsb, lane, y0, y1);  // not asked about `landed` yet: as in run_phase
         __syncwarp();  // every lane is done with the buffer
-        if (tile + nw < r1) issue(tile + nw);
+        ok = landed;
+        if (ok && tile + nw < r1) issue(tile + nw);
         const int pair = s_pair[t];
-        if (pair >= 0) {
+        if (ok && pair >= 0) {
           float *y = p.Y + (size_t)pair * H + (tile - job * tiles) * 16 + g;
           y[0] = y0;
           y[8] = y1;
@@ -423,6 +432,8 @@ __device__ __noinline__ void stage_down_q6k(const StackParams &p, const LayerDes
       }
     }
   }
+  parity_io = parity;
+  ok_io = ok;
   __syncthreads();  // the ring area returns to the projection phases
 }
 
@@ -450,10 +461,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_stack_kernel(const StackParam
   const q4e::JobTable jt{jbase, uexp};
 
   if (lane == 0)
-    for (int s = 0; s < q4e::kMaxStages; ++s) mbar_init(&sm.bars[warp * q4e::kMaxStages + s], 1);
-  if (threadIdx.x == 0) {
-    *s_fail = 0;
-  }
+    for (int s = 0; s < q4e::kMaxStages; ++s) mbar_init(&sm.bars[warp * q4e::kMaxStages + s], c == 0 && s == 0 && warp + 1 == p.stall_copy ? 2 : 1);
+  if (threadIdx.x == 0) *s_fail = 0;
   mbar_init_fence();
   __syncthreads();
 
@@ -494,7 +503,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_stack_kernel(const StackParam
     KNJ_STAMP(1);
     arrivals += G;
     grid_arrive(p.sync);
-    if (!grid_wait(p.sync, arrivals + (l == 0 ? (unsigned)p.stall : 0u), p.wait_cycles)) return;
+    if (!grid_wait(p.sync, s_fail, arrivals + (l == 0 ? (unsigned)p.stall : 0u), p.wait_cycles)) return;
     KNJ_STAMP(2);
 
     // ---- stage 2: top-k per token (every CTA for itself), the per-expert token sets, the job table
@@ -545,7 +554,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_stack_kernel(const StackParam
     KNJ_STAMP(4);
     arrivals += G;
     grid_arrive(p.sync);
-    if (!grid_wait(p.sync, arrivals, p.wait_cycles)) return;
+    if (!grid_wait(p.sync, s_fail, arrivals, p.wait_cycles)) return;
     KNJ_STAMP(5);
 
     // ---- stage 4: down -> Y (one row per pair)
@@ -568,7 +577,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_stack_kernel(const StackParam
     KNJ_STAMP(6);
     arrivals += G;
     grid_arrive(p.sync);
-    if (!grid_wait(p.sync, arrivals, p.wait_cycles)) return;
+    if (!grid_wait(p.sync, s_fail, arrivals, p.wait_cycles)) return;
     KNJ_STAMP(7);
 
     // ---- stage 5: ordered weighted sum of a token's k rows, residual last, four columns per thread
@@ -612,11 +621,10 @@ __global__ void __launch_bounds__(kThreads, 1) moe_stack_kernel(const StackParam
     if (l + 1 < p.n_layers) {
       arrivals += G;
       grid_arrive(p.sync);
-      if (!grid_wait(p.sync, arrivals, p.wait_cycles)) return;
+      if (!grid_wait(p.sync, s_fail, arrivals, p.wait_cycles)) return;
     }
     KNJ_STAMP(9);
   }
-  if (!ok && threadIdx.x == 0) atomicExch(p.sync + 1, 1u);
 }
 
 }  // namespace
@@ -788,6 +796,12 @@ int knj_moe_stack_set_wait(knj_moe_stack *st, long long wait_cycles, int stall_f
   st->p.wait_cycles = wait_cycles > 0 ? wait_cycles : kMaxWaitCycles;
   st->p.stall = stall_first_barrier > 0 ? stall_first_barrier : 0;
   if (st->small) small_stack_set_wait(st->small, st->p.wait_cycles, st->p.stall);
+  return KNJ_OK;
+}
+
+int knj_moe_stack_test_stall_copy(knj_moe_stack *st, int warp) {
+  KNJ_REQUIRE(st && !st->small && warp < q4e::kWarps, "knj_moe_stack_test_stall_copy: no such warp, or a stack without such copies");
+  st->p.stall_copy = warp >= 0 ? warp + 1 : 0;
   return KNJ_OK;
 }
 

@@ -230,6 +230,41 @@ def test_bounded_wait_gives_up_and_the_stack_recovers():
     st.close()
 
 
+@pytest.mark.parametrize("down", ["q4k", "q6k"])
+@pytest.mark.parametrize("warp", [0, 2, 9])
+def test_a_copy_that_does_not_land_is_reported_whichever_warp_waits(down, warp):
+    """The first weight copies of one warp of CTA 0 never count as landed: status() reports KNJ_E_TIMEOUT although the CTA's
+    other warps land theirs, and the next normal launch is right again. Jobs of 32 gate+up tiles and 112 down tiles, 14 to
+    41 of them over 148 CTAs: warps 0 and 2 already wait in the gate+up phase (3 to 8 tiles a CTA), warp 9 in the down
+    phase alone (10 and more)."""
+    from kanjoos_b200 import _lib
+    from kanjoos_b200.moe import ExpertBank, FusedMoeStack
+    E, H, F, T, k = 16, 1792, 256, 8, 8
+    bank = synth.expert_bank(812, 0, n_experts=E, hidden=H, ffn=F)
+    if down == "q6k":
+        bank = dict(bank, down=_q6k_down(812, E, H, F))
+    wr, _ = synth.router_weight(812, 0, n_experts=E, hidden=H)
+    b = ExpertBank.from_numpy(bank, wr, None, synth.norm_weight(812, 0, H))
+    x = dev(synth.hidden_rows(812, T, H))
+    st = FusedMoeStack([b], top_k=k, n_tokens=T, dtype=torch.float32, taps=True)
+    want = st.step(x).clone()
+    st.status()
+    jobs = int(((torch.bincount(st.taps[0][0].long(), minlength=E) + 3) // 4).sum())
+    assert 14 <= jobs <= 41
+    st.set_wait(wait_cycles=2_000_000)   # about a millisecond
+    _lib.check(_lib.lib().knj_moe_stack_test_stall_copy(st._h, warp))
+    st.step(x)
+    with pytest.raises(_lib.KnjError) as ei:
+        st.status()
+    assert ei.value.code == -5
+    st.set_wait(0)
+    _lib.check(_lib.lib().knj_moe_stack_test_stall_copy(st._h, -1))
+    got = st.step(x)
+    st.status()
+    assert torch.equal(got, want)
+    st.close()
+
+
 def test_refusals():
     from kanjoos_b200.moe import FusedMoeStack
     banks, _ = _banks(803, 1, 16, 512, 256)
