@@ -409,7 +409,7 @@ typedef struct knj_moe_ffn_args {
   int32_t *tap_pair_exp;     /* [T*k] */
   float *tap_pair_w;         /* [T*k] */
   /* format of w_down: 0 = Q4_K as above, 1 = Q6_K [E][hidden][ffn/256][210] (the
-   * mixed-format layers of Q4_K_M checkpoints; the prefill launch takes them for ffn <= 1024) */
+   * mixed-format layers of Q4_K_M checkpoints; the prefill launch and the whole-stack launch take them for ffn <= 1024) */
   int32_t down_format;
   /* prefill launch: 0 = per-pair rows + the ordered combine kernel (bit-reproducible, the CPU path's summation
    * order; the faster form on B200 at every measured size); 1 = the weighted combine fused into the down GEMM's

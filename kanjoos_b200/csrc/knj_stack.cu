@@ -41,6 +41,7 @@ constexpr int kMaxT = 64;  // tokens per step
 constexpr int kThreads = q4e::kWarps * 32;
 constexpr int kSplitMaxT = 16;  // batches up to this size may split a tile's K range over several warps
 constexpr int kMaxSlices = 8;  // hidden <= 2048: the logits keep a router row in registers
+constexpr int kMaxF6 = 1024;   // ffn of layers with Q6_K down matrices: as the prefill launch takes them, and as far as it is tested
 
 struct LayerMaps {  // stay in global memory: the TMA unit reads them there
   CUtensorMap mg, mu, md;  // gate, up, down weights as TMA boxes of the projection phases
@@ -139,6 +140,16 @@ __host__ __device__ inline Plan make_plan(const q4e::PhaseShape &gu, const q4e::
   pl.red = T <= kSplitMaxT ? take((size_t)q4e::kWarps * 32 * sizeof(float4)) : 0;
   pl.total = o;
   return pl;
+}
+
+// Warps that take tiles in a Q6_K down phase: each needs a buffer for one whole tile, which lie in the ring and panel areas
+// (the phase engine is idle) in front of the phase's own panel. Three superblocks a row (ffn 768) leave room for 14 warps at
+// hidden 512 and 16 at hidden 2048, four for 11 and 12. 0: the areas do not hold a panel and one tile.
+__host__ __device__ inline int down6_warps(const Plan &pl, int nsb) {
+  const size_t room = pl.bars - pl.ring, panel = q6b::tile_panel_bytes(nsb);
+  if (room < panel) return 0;
+  const int fit = (int)((room - panel) / q6b::tile_bytes(nsb));
+  return fit < q4e::kWarps ? fit : q4e::kWarps;
 }
 
 __device__ __forceinline__ void load8_bf16(const __nv_bfloat16 *p, float (&v)[8]) {
@@ -360,7 +371,7 @@ __device__ __noinline__ void stage_plan(const StackParams &p, const LayerDesc &L
 
 // Down phase of a layer whose down matrices are Q6_K: the CTA's run of the flat (job, 16-row tile) list, as in the Q4_K
 // engine, with q6b's whole tiles: a warp copies a tile of its own (10 KB at ffn 768), multiplies it and asks for the next.
-// The buffers lie in the ring area and the panel behind them; where sixteen do not fit (ffn 1024) fewer warps take tiles.
+// The buffers lie in the ring area and the panel behind them; where sixteen do not fit fewer warps take tiles (down6_warps).
 // Before, blocks of 64 rows were staged and reduced by the whole CTA, three CTA barriers each: 45 us on the mean and 60 to
 // the last CTA at 8 tokens (51 experts, 66 MB, 10 us of HBM time), where the Q4_K phase takes 18.
 __device__ __noinline__ void stage_down_q6k(const StackParams &p, const LayerDesc &L, const Plan &pl, uint8_t *smem, unsigned &parity_io,
@@ -374,7 +385,7 @@ __device__ __noinline__ void stage_down_q6k(const StackParams &p, const LayerDes
   int *s_pair = reinterpret_cast<int *>(smem + pl.pair);
   volatile int *fail = reinterpret_cast<volatile int *>(smem + pl.fail);
   const uint32_t tb = (uint32_t)q6b::tile_bytes(nsb);
-  const int nw = min(q4e::kWarps, (int)((pl.bars - pl.ring - (uint32_t)q6b::tile_panel_bytes(nsb)) / tb));
+  const int nw = down6_warps(pl, nsb);
   uint8_t *buf = smem + pl.ring + (size_t)warp * tb, *panel = smem + pl.ring + (size_t)nw * tb;
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem + pl.bars) + warp * q4e::kMaxStages;
   static_assert(q6b::kTileTok == q4e::kJobTok, "one job table");
@@ -664,6 +675,7 @@ int knj_moe_stack_create(const knj_moe_ffn_args *layers, int n_layers, knj_moe_s
   KNJ_REQUIRE(H > 0 && H % 256 == 0 && H <= 256 * kMaxSlices, "knj_moe_stack_create: hidden=%d must be a multiple of 256, at most %d", H,
               256 * kMaxSlices);
   KNJ_REQUIRE(F > 0 && F % 256 == 0 && F <= 4096, "knj_moe_stack_create: ffn=%d must be a multiple of 256, at most 4096", F);
+  KNJ_REQUIRE(!any_q6k || F <= kMaxF6, "knj_moe_stack_create: ffn=%d: layers with Q6_K down matrices are taken up to ffn %d", F, kMaxF6);
   KNJ_REQUIRE(k >= 1 && k <= 8 && k <= E && E <= 256, "knj_moe_stack_create: top_k=%d / n_experts=%d out of range", k, E);
   StackParams sp{};
   sp.gu.N = F; sp.gu.nsb = H / 256; sp.gu.sbs = (sp.gu.nsb % 2 == 0) ? 2 : 1; sp.gu.tiles = F / 8;
@@ -724,11 +736,8 @@ int knj_moe_stack_create(const knj_moe_ffn_args *layers, int n_layers, knj_moe_s
     else --sp.gu.stages;
   }
   const size_t smem = total();
-  if (any_q6k) {  // a Q6_K down phase stages a 64-row block and eight activation rows in the ring area
-    const size_t need = q6b::block_bytes(F) + q6b::act_scratch_bytes(F, q4e::kWarps);
-    const size_t ring = std::max(q4e::phase_ring_bytes(sp.gu.sbs, sp.gu.stages), q4e::phase_ring_bytes(sp.dn.sbs, sp.dn.stages));
-    KNJ_REQUIRE(need <= ring, "knj_moe_stack_create: ffn=%d is too long for the Q6_K down phase's staging (%zu > %zu bytes)", F, need, ring);
-  }
+  KNJ_REQUIRE(!any_q6k || down6_warps(make_plan(sp.gu, sp.dn, T, k), sp.dn.nsb) >= 1,
+              "knj_moe_stack_create: ffn=%d leaves no room for a tile of the Q6_K down phase", F);
   if (!prop.cooperativeLaunch || smem > (size_t)prop.sharedMemPerBlockOptin) {
     set_error("knj_moe_stack_create: the device lacks cooperative launch or %zu bytes of shared memory per block", smem);
     return KNJ_E_REFUSE;

@@ -286,6 +286,18 @@ def test_stack_create_refuses_bad_arguments(L):
     L.knj_moe_stack_destroy(None)
 
 
+@pytest.mark.parametrize("ffn,what", [(1280, b"up to ffn 1024"), (4096, b"up to ffn 1024"), (1024, b"null tensor pointer")])
+def test_stack_create_refuses_long_q6k_rows_by_their_length(L, ffn, what):
+    """Q6_K down matrices are taken up to ffn 1024, and that is what the refusal says; at 1024 the next check answers."""
+    from kanjoos_b200._lib import MoeFfnArgs
+    a = MoeFfnArgs()
+    a.n_tokens, a.hidden, a.ffn, a.n_experts, a.top_k = 4, 2048, ffn, 16, 4
+    a.ldx = a.ldo = 2048
+    a.down_format = 1
+    h = C.c_void_p()
+    assert L.knj_moe_stack_create(C.byref(a), 1, C.byref(h)) == -1 and what in L.knj_last_error_string()
+
+
 def _run_ref_binary(name):
     import subprocess
     exe = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "oracle", "_ref", name)
