@@ -173,6 +173,35 @@ def test_q6k_down_phase_follows_the_layer_launch_at_every_row_length(F, T):
     assert report(got, want, f"Q6_K down phase, ffn {F}, T={T}")["rel_rmse"] <= 1e-5
 
 
+@pytest.mark.parametrize("F,T,E", [(768, 8, 32), (768, 64, 16), (1024, 8, 16), (1024, 64, 32)])
+def test_q6k_down_phase_with_more_tiles_than_warps(F, T, E):
+    """At hidden 2048 a CTA has more tiles than warps that take them (128 tiles a job, 16 at ffn 768 and 12 at ffn 1024), so a
+    warp copies tile after tile into its one buffer; a Q4_K layer between two Q6_K layers hands the barriers' phases and the
+    ring area over both ways. Against the layer launches, f32 stream: nothing but summation order may differ."""
+    from kanjoos_b200.moe import ExpertBank, FusedMoeStack, MoeStack
+    L, H, k = 3, 2048, 8
+    banks = []
+    for l in range(L):
+        bank = synth.expert_bank(813, l, n_experts=E, hidden=H, ffn=F)
+        if l != 1:
+            bank = dict(bank, down=_q6k_down(813 + l, E, H, F))
+        wr, _ = synth.router_weight(813, l, n_experts=E, hidden=H)
+        banks.append(ExpertBank.from_numpy(bank, wr, None, synth.norm_weight(813, l, H)))
+    x = dev(synth.hidden_rows(813, T, H))
+    ref = MoeStack(banks, top_k=k, max_tokens=T).step(x).cpu().numpy()
+    st = FusedMoeStack(banks, top_k=k, n_tokens=T, dtype=torch.float32, taps=True)
+    got = st.step(x).cpu().numpy()
+    st.status()
+    for l in (0, 2):
+        jobs = int(((torch.bincount(st.taps[l][0].flatten().long(), minlength=E) + 3) // 4).sum())
+        assert jobs * (H // 16) > (16 if F == 768 else 12) * torch.cuda.get_device_properties(0).multi_processor_count, jobs
+    assert np.array_equal(got, st.step(x).cpu().numpy())
+    st.status()
+    st.close()
+    s = report(got, ref, f"Q6_K down phase of several tiles a warp, ffn {F}, T={T}")
+    assert s["unwritten"] == 0 and s["rel_rmse"] <= 1e-5
+
+
 @pytest.mark.parametrize("B", [1, 8, 64])
 def test_config4_full_size_stack_checked_layers(B):
     """Config 4: the 48-layer resident stack at full size (about 15 GiB of random-init Q4_K experts), f32 residual
