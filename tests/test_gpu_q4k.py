@@ -172,6 +172,37 @@ def test_a_wait_that_gives_up_leaves_nan(m, n_out, nan_rows):
     assert torch.equal(y, want)
 
 
+@pytest.mark.parametrize("m,n_in,n_out,nan_rows", [
+    (17, 1024, 8192, 8),   # three jobs of eight (five of four: 2560 tiles), the last of one row; the first block's tiles are rows 0..7's
+    (9, 4096, 4096, 8),    # two jobs (three of four: 768 tiles of sixteen superblocks), K split over the warps of a tile
+])
+def test_a_wait_that_gives_up_leaves_nan_in_jobs_of_eight(m, n_in, n_out, nan_rows):
+    """The same for 16-bit rows in jobs of eight: NaN in all eight rows of a given-up tile, in no row behind the last, and
+    everything else right."""
+    from kanjoos_b200 import _lib, ops
+    L = _lib.lib()
+    rng = np.random.Generator(np.random.Philox([m, n_out]))
+    W = dev(synth.q4k_rows(rng, n_out, n_in))
+    x = dev(rng.standard_normal((m, n_in)).astype(np.float32)).to(torch.bfloat16)
+    want = ops.q4k_matmul(W, x)
+    guard = torch.full((m + 8, n_out), SENTINEL, dtype=torch.float32, device="cuda")
+    y = guard[:m]
+    L.knj_decode_wait_limit(2_000_000)
+    L.knj_q4k_matmul_test_stall(1)
+    try:
+        product_into(W, x, y)
+        torch.cuda.synchronize()
+    finally:
+        L.knj_q4k_matmul_test_stall(0)
+        L.knj_decode_wait_limit(0)
+    bad = torch.isnan(y)
+    assert bad[:nan_rows, :16].all() and not bad[nan_rows:, :16].any()
+    assert not (y == SENTINEL).any() and int(bad.sum()) < y.numel() // 16
+    assert torch.equal(y[~bad], want[~bad]) and (guard[m:] == SENTINEL).all()
+    product_into(W, x, y)
+    assert torch.equal(y, want)
+
+
 def test_refusals_do_not_launch():
     from kanjoos_b200 import _lib, ops
     W = torch.zeros((16, 1, 144), dtype=torch.uint8, device="cuda")
