@@ -277,7 +277,7 @@ __device__ __forceinline__ void tile_part(const uint8_t *stage, int pitch, int w
   const float ng = __half2float(__ushort_as_half((unsigned short)(hg.x >> 16))) * 64.0f;
   const float dh = __half2float(__ushort_as_half((unsigned short)(hh.x & 0xffffu))) * 16777216.0f;
   const float nh = __half2float(__ushort_as_half((unsigned short)(hh.x >> 16))) * 64.0f;
-  if (PL == 1) {
+  if constexpr (PL == 1) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       float sg = 0.f, sh = 0.f;
@@ -289,18 +289,18 @@ __device__ __forceinline__ void tile_part(const uint8_t *stage, int pitch, int w
       rg[i] = dg * sg - ng * cm[0][i];
       rh[i] = dh * sh - nh * cm[0][2 + i];
     }
-    return;
-  }
+  } else {
 #pragma unroll
-  for (int q = 0; q < NG; ++q) {
-    float sg = 0.f, sh = 0.f;
+    for (int q = 0; q < NG; ++q) {
+      float sg = 0.f, sh = 0.f;
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      sg += (ce[q][c][0] + ce[q][c][1]) + (co[q][c][0] + co[q][c][1]);
-      sh += (ce[q][c][2] + ce[q][c][3]) + (co[q][c][2] + co[q][c][3]);
+      for (int c = 0; c < NC; ++c) {
+        sg += (ce[q][c][0] + ce[q][c][1]) + (co[q][c][0] + co[q][c][1]);
+        sh += (ce[q][c][2] + ce[q][c][3]) + (co[q][c][2] + co[q][c][3]);
+      }
+      rg[q] = dg * sg - ng * (cm[q][0] + cm[q][1]);
+      rh[q] = dh * sh - nh * (cm[q][2] + cm[q][3]);
     }
-    rg[q] = dg * sg - ng * (cm[q][0] + cm[q][1]);
-    rh[q] = dh * sh - nh * (cm[q][2] + cm[q][3]);
   }
 }
 
