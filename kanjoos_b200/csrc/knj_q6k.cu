@@ -21,9 +21,9 @@ using namespace knj;
 namespace {
 
 constexpr int kQ6Tok = q6b::kTok;     // tokens per pass
-constexpr int kQ6Rows = q6b::kRows;   // output rows per staged block
-constexpr int kQ6MaxSub = 1;          // blocks per work item (the activation side is prepared once per item): with two CTAs
-                                      // per SM two or four blocks per item measured no faster (118 us at batch 64 either way)
+constexpr int kQ6Rows = q6b::kRows;   // output rows per staged block, one block per work item: with two CTAs per SM two or
+                                      // four blocks per item (the activation side prepared once) measured no faster (118 us
+                                      // at batch 64 either way)
 constexpr int kQ6Threads = 256;  // two CTAs per SM: one's block travels while the other computes
 
 struct Q6Params {
@@ -35,42 +35,37 @@ struct Q6Params {
   int64_t idxStride;
   int *status;  // raised when the bounded wait for a weight block gave up (may be null)
   long long wait_cycles;
-  int two_blocks;  // the shared memory holds two weight blocks (the next one travels while this one is worked on)
 };
 
 __global__ void __launch_bounds__(kQ6Threads, 2) q6k_proj_kernel(const Q6Params p) {
-  extern __shared__ __align__(16) uint8_t s_raw[];  // weight block(s), then the activation side (q6b::carve)
+  extern __shared__ __align__(16) uint8_t s_raw[];  // weight block, then the activation side (q6b::carve)
   __shared__ int s_pair[kQ6Tok];
-  __shared__ uint64_t s_bars[2];  // the weight blocks' bulk copies
+  __shared__ uint64_t s_bar;  // the weight blocks' bulk copies
   __shared__ int s_fail;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
-    mbar_init(&s_bars[0], 1);
-    mbar_init(&s_bars[1], 1);
+    mbar_init(&s_bar, 1);
     s_fail = 0;
     mbar_init_fence();
   }
   const int row_bytes = p.K / KNJ_QK_K * KNJ_Q6K_BYTES;
-  const q6b::Bufs b = q6b::carve(s_raw, p.K, kQ6Threads / 32, p.two_blocks != 0, s_bars, &s_fail);
+  const q6b::Bufs b = q6b::carve(s_raw, p.K, kQ6Threads / 32, &s_bar, &s_fail);
   const int blocks = (p.N + kQ6Rows - 1) / kQ6Rows;
   const int n_act = p.n_active[0];
-  // blocks per item: as many as leave every CTA about two items (few experts: one block per item)
-  const int sub = max(1, min(kQ6MaxSub, n_act * blocks / (2 * (int)gridDim.x)));
-  const int chunks = (blocks + sub - 1) / sub;
-  const int total = n_act * chunks;
+  const int total = n_act * blocks;
   const bool bulk = (reinterpret_cast<uintptr_t>(p.W) & 15u) == 0 && p.N % kQ6Rows == 0;
   unsigned staged = 0;  // bulk copies waited for so far
   for (int it = blockIdx.x; it < total; it += gridDim.x) {
-    const int a = it / chunks, chunk = it - a * chunks;
+    const int a = it / blocks, block = it - a * blocks;
     const int e = p.exp_list[a];
     const int cnt = p.pair_cnt[e];
-    const int n0 = chunk * sub * kQ6Rows, n_rows = min(sub * kQ6Rows, p.N - n0);
+    const int n0 = block * kQ6Rows, n_rows = min(kQ6Rows, p.N - n0);
     for (int tok0 = 0; tok0 < cnt; tok0 += kQ6Tok) {
       const int nt = min(kQ6Tok, cnt - tok0);
       __syncthreads();  // the previous pass is done with the shared buffers
       if ((int)threadIdx.x < kQ6Tok) s_pair[threadIdx.x] = (int)threadIdx.x < nt ? p.pair_idx[(size_t)e * p.idxStride + tok0 + threadIdx.x] : -1;
       __syncthreads();
-      if (!q6b::chunk_pass<kQ6Threads / 32>(b, p.W + ((size_t)e * p.N + n0) * row_bytes, n_rows, p.K, p.A, p.Y + n0, p.N, s_pair, nt, staged,
+      if (!q6b::block_pass<kQ6Threads / 32>(b, p.W + ((size_t)e * p.N + n0) * row_bytes, n_rows, p.K, p.A, p.Y + n0, p.N, s_pair, nt, staged,
                                             bulk, p.wait_cycles, lane, warp)) {
         if (threadIdx.x == 0 && p.status) atomicExch(p.status, 1);  // a copy that never completed: report and leave
         return;
@@ -88,9 +83,7 @@ int knj_q6k_proj_launch(const float *A, const uint8_t *W6, const int32_t *pair_i
                         int n_experts, int *status, knj_stream_t s) {
   KNJ_REQUIRE(A && W6 && pair_idx && pair_cnt && exp_list && n_active && Y, "knj_q6k_proj: null pointer");
   KNJ_REQUIRE(K > 0 && K % 256 == 0 && N > 0 && n_experts > 0, "knj_q6k_proj: K=%d must be a multiple of 256, N=%d positive", K, N);
-  const size_t one = q6b::block_bytes(K) + q6b::act_scratch_bytes(K, kQ6Threads / 32);
-  const bool two = false;  // one block buffer per CTA and two CTAs per SM measured faster than one CTA with two buffers
-  const size_t smem = one + (two ? q6b::block_bytes(K) : 0);
+  const size_t smem = q6b::block_bytes(K) + q6b::act_scratch_bytes(K, kQ6Threads / 32);
   KNJ_REQUIRE(smem <= 220 * 1024, "knj_q6k_proj: K=%d is too long for the staged rows", K);
   KNJ_REQUIRE(aligned16(A) && K % 4 == 0, "knj_q6k_proj: activation rows must be 16-byte aligned");
   int dev = 0;
@@ -101,7 +94,7 @@ int knj_q6k_proj_launch(const float *A, const uint8_t *W6, const int32_t *pair_i
     KNJ_CUDA(cudaFuncSetAttribute(q6k_proj_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     opted[dev] = smem;
   }
-  Q6Params p{A, W6, pair_idx, pair_cnt, exp_list, n_active, Y, N, K, idxStride, status, knj::decode_wait_cycles(), two ? 1 : 0};
+  Q6Params p{A, W6, pair_idx, pair_cnt, exp_list, n_active, Y, N, K, idxStride, status, knj::decode_wait_cycles()};
   const long long items = (long long)n_experts * ((N + kQ6Rows - 1) / kQ6Rows);
   const long long per_sm = smem + 1024 <= 113 * 1024 ? 2 : 1;
   const long long cap = (long long)sm_count() * per_sm;

@@ -1,7 +1,9 @@
 // knj_q6k_block.cuh -- decode-class arithmetic over a block of Q6_K rows staged in shared memory (210-byte
 // superblocks: 128 B low nibbles, 64 B high bit pairs, 16 int8 scales, fp16 d; w = d * sc * (q - 32); decoders
-// kernels/knj_q4k.h:170-196, CPU dot_q6_k src/loader/dequant.cpp:986-1022). Shared by the stand-alone projection
-// kernel (knj_q6k.cu) and the down phase of the whole-stack launch (knj_stack.cu), so both produce the same bits.
+// kernels/knj_q4k.h:170-196, CPU dot_q6_k src/loader/dequant.cpp:986-1022). Two forms of the same fragments: blocks of
+// 64 rows for the whole CTA (the stand-alone projection, knj_q6k.cu) and whole tiles of 16 rows per warp (the down phase of
+// the whole-stack launch, knj_stack.cu). They split K and scale the activations differently, so they agree to f32 rounding
+// (1e-7), not to the bit.
 #pragma once
 #include "knj_common.cuh"
 #include "knj_q4k.h"
@@ -23,11 +25,8 @@ __device__ __forceinline__ void stage_block(uint8_t *wbuf, const uint8_t *src, i
 }
 
 // The same by one bulk copy that completes on `bar` (one thread calls it; the others wait on the barrier): for blocks
-// that start on a 16-byte boundary and are a multiple of 16 bytes long (bulk_ok). Earlier reads of the buffer by
+// that start on a 16-byte boundary and are a multiple of 16 bytes long. Earlier reads of the buffer by
 // this CTA must have been ordered before the call by a CTA barrier.
-__device__ __forceinline__ bool bulk_ok(const uint8_t *src, int bytes) {
-  return ((reinterpret_cast<uintptr_t>(src) | (uintptr_t)bytes) & 15u) == 0;
-}
 __device__ __forceinline__ void stage_block_bulk(uint8_t *wbuf, const uint8_t *src, int bytes, uint64_t *bar) {
   fence_proxy_async();
   mbar_expect_tx(bar, (uint32_t)bytes);
@@ -43,36 +42,34 @@ __device__ __forceinline__ void stage_block_bulk(uint8_t *wbuf, const uint8_t *s
 // is permuted so that lane t of a fragment row owns four consecutive codes (one 32-bit word of low nibbles, one of
 // high bit pairs): MMA columns (2t, 2t+1, 2t+8, 2t+9) stand for weights 4t .. 4t+3, on both operands.
 //
-// Shared memory of a caller (Bufs): one or two weight-block buffers, the pass's f32 activation rows, the
-// B fragments of every k-step ([K/16][2][32] x 8 bytes, built once per expert and token pass and used by every
-// row block of the expert), the partial sums of the warps that share a 16-row tile ([4 tiles][WARPS/4][2][2][32]
-// f32), the kTok inverse scales and scales, two mbarriers for the blocks' bulk copies.
+// Shared memory of a caller (Bufs): the weight-block buffer, the pass's f32 activation rows, the
+// B fragments of every k-step ([K/16][2][32] x 8 bytes, built once per pass), the partial sums of the warps that share a
+// 16-row tile ([4 tiles][WARPS/4][2][2][32] f32), the kTok inverse scales and scales, one mbarrier for the blocks' bulk
+// copies. (A second buffer, for the next block to travel meanwhile, measured slower than two CTAs per SM with one each.)
 __host__ __device__ inline size_t block_bytes(int K) { return ((size_t)kRows * (K / KNJ_QK_K) * KNJ_Q6K_BYTES + 15) & ~(size_t)15; }
 __host__ __device__ inline size_t panel_bytes(int K) { return (size_t)(K / 16) * 2 * 32 * 8; }
 __host__ __device__ inline size_t red_bytes(int warps) { return (size_t)4 * (warps / 4) * 2 * 2 * 32 * 4; }
-// bytes behind the weight-block buffer(s): the pass's activation rows, panel, partial sums, scales
+// bytes behind the weight-block buffer: the pass's activation rows, panel, partial sums, scales
 __host__ __device__ inline size_t act_scratch_bytes(int K, int warps) {
   return (size_t)kTok * K * 4 + panel_bytes(K) + red_bytes(warps) + 2 * kTok * 4;
 }
 
 struct Bufs {
-  uint8_t *w[2];   // weight blocks (w[1] == w[0]: no double buffering)
-  float *abuf;     // [kTok][K] f32: the pass's activation rows
+  uint8_t *w;     // weight block
+  float *abuf;    // [kTok][K] f32: the pass's activation rows
   uint2 *panel;
   float *red, *inv;
-  uint64_t *bars;  // [2], initialised by the caller with one arrival each
-  int *fail;       // shared flag a wait that gives up raises
+  uint64_t *bar;  // initialised by the caller with one arrival
+  int *fail;      // shared flag a wait that gives up raises
 };
-__device__ __forceinline__ Bufs carve(uint8_t *base, int K, int warps, bool two_blocks, uint64_t *bars, int *fail) {
+__device__ __forceinline__ Bufs carve(uint8_t *base, int K, int warps, uint64_t *bar, int *fail) {
   Bufs b;
-  b.w[0] = base;
-  b.w[1] = two_blocks ? base + block_bytes(K) : base;
-  uint8_t *p = base + (two_blocks ? 2 : 1) * block_bytes(K);
-  b.abuf = reinterpret_cast<float *>(p);
-  b.panel = reinterpret_cast<uint2 *>(p + (size_t)kTok * K * 4);
+  b.w = base;
+  b.abuf = reinterpret_cast<float *>(base + block_bytes(K));
+  b.panel = reinterpret_cast<uint2 *>(b.abuf + (size_t)kTok * K);
   b.red = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(b.panel) + panel_bytes(K));
   b.inv = b.red + red_bytes(warps) / 4;
-  b.bars = bars;
+  b.bar = bar;
   b.fail = fail;
   return b;
 }
@@ -227,53 +224,34 @@ __device__ __forceinline__ void block_mma(const uint8_t *wbuf, const Bufs &b, in
 }
 
 // One pass of up to kTok activation rows (row t = A + rows_of[t] * K in global memory; rows_of in shared memory)
-// over n_rows consecutive weight rows of one expert starting at src (a multiple of 64 rows into the expert's
-// matrix), 64 at a time: Y[rows_of[t] * ldy + r] = the sum for weight row r < n_rows. `bulk`: the blocks travel as
-// bulk copies, the next one under way while this one is worked on when b holds two buffers; `staged` counts the
-// bulk copies this CTA has waited for (buffer = staged & 1, barrier phase = staged >> 1 & 1). Every thread of the
-// CTA calls it with the same arguments; the caller puts a CTA barrier between two calls. False: a wait gave up.
+// over one block of n_rows <= kRows consecutive weight rows of one expert starting at src (a multiple of 64 rows into the
+// expert's matrix): Y[rows_of[t] * ldy + r] = the sum for weight row r < n_rows. `bulk`: the block travels as one bulk copy
+// while the activation side is prepared; `staged` counts the bulk copies this CTA has waited for (barrier phase =
+// staged & 1). Every thread of the CTA calls it with the same arguments; the caller puts a CTA barrier between two calls.
+// False: a wait gave up.
 template <int WARPS>
-__device__ __forceinline__ bool chunk_pass(const Bufs &b, const uint8_t *src, int n_rows, int K, const float *A, float *Y, int ldy,
+__device__ __forceinline__ bool block_pass(const Bufs &b, const uint8_t *src, int n_rows, int K, const float *A, float *Y, int ldy,
                                            const int *rows_of, int nt, unsigned &staged, bool bulk, long long wait_cycles, int lane,
                                            int warp) {
   const int tid = warp * 32 + lane, row_bytes = K / KNJ_QK_K * KNJ_Q6K_BYTES;
-  const int nsub = (n_rows + kRows - 1) / kRows;
-  const bool two = b.w[1] != b.w[0];
-  // the first block travels while the activation side is prepared
-  if (bulk && tid == 0) stage_block_bulk(b.w[two ? (staged & 1u) : 0], src, min(kRows, n_rows) * row_bytes, &b.bars[staged & 1u]);
+  if (bulk && tid == 0) stage_block_bulk(b.w, src, n_rows * row_bytes, b.bar);
   for (int i = tid; i < nt * (K / 4); i += WARPS * 32) {
     const int t = i / (K / 4), k4 = i - t * (K / 4);
     reinterpret_cast<float4 *>(b.abuf + (size_t)t * K)[k4] = __ldcg(reinterpret_cast<const float4 *>(A + (size_t)rows_of[t] * K) + k4);
   }
   __syncthreads();
   prepare_panel<WARPS>(b, K, nt, lane, warp);
-  for (int sub = 0; sub < nsub; ++sub) {
-    const int r0 = sub * kRows, nr = min(kRows, n_rows - r0);
-    const uint8_t *wbuf;
-    if (bulk) {
-      wbuf = b.w[two ? (staged & 1u) : 0];
-      const bool landed = mbar_wait_for(&b.bars[staged & 1u], (staged >> 1) & 1u, wait_cycles, b.fail);
-      ++staged;
-      // also: every warp is done with the previous block (and with the partial sums of its reduction)
-      if (!__syncthreads_and(landed)) return false;
-      if (sub + 1 < nsub && two && tid == 0)
-        stage_block_bulk(b.w[staged & 1u], src + (size_t)(r0 + kRows) * row_bytes, min(kRows, n_rows - r0 - kRows) * row_bytes,
-                         &b.bars[staged & 1u]);
-    } else {
-      __syncthreads();
-      stage_block(b.w[0], src + (size_t)r0 * row_bytes, nr * row_bytes, tid, WARPS * 32);
-      __syncthreads();
-      wbuf = b.w[0];
-    }
-    auto store = [&](int r, int t, float v) { Y[(size_t)rows_of[t] * ldy + r0 + r] = v; };
-    if (nt <= 4) block_mma<1, WARPS>(wbuf, b, K, nr, nt, lane, warp, store);
-    else block_mma<2, WARPS>(wbuf, b, K, nr, nt, lane, warp, store);
-    if (bulk && !two && sub + 1 < nsub) {  // one buffer: the next block can only start once this one is done with
-      __syncthreads();
-      if (tid == 0)
-        stage_block_bulk(b.w[0], src + (size_t)(r0 + kRows) * row_bytes, min(kRows, n_rows - r0 - kRows) * row_bytes, &b.bars[staged & 1u]);
-    }
+  if (bulk) {
+    const bool landed = mbar_wait_for(b.bar, staged & 1u, wait_cycles, b.fail);
+    ++staged;
+    if (!__syncthreads_and(landed)) return false;
+  } else {
+    stage_block(b.w, src, n_rows * row_bytes, tid, WARPS * 32);
+    __syncthreads();
   }
+  auto store = [&](int r, int t, float v) { Y[(size_t)rows_of[t] * ldy + r] = v; };
+  if (nt <= 4) block_mma<1, WARPS>(b.w, b, K, n_rows, nt, lane, warp, store);
+  else block_mma<2, WARPS>(b.w, b, K, n_rows, nt, lane, warp, store);
   return true;
 }
 
