@@ -363,7 +363,6 @@ __device__ __noinline__ void stage_plan(const StackParams &p, const LayerDesc &L
       }
       __syncwarp();
       q4e::job_prefix(jbase, lane);
-      if (lane == 0) jbase[259] = total;  // active experts (behind the job table, inside its padding)
     }
     __syncthreads();
 
