@@ -188,12 +188,6 @@ __device__ __forceinline__ bool mbar_wait_for(uint64_t *bar, uint32_t parity, lo
   }
 }
 
-// The same with one answer for the warp, whose lanes all call it. Each lane times its wait for itself: one could give up
-// just before the copy lands for the others, and they are about to meet in warp-wide instructions.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, long long limit_cycles, volatile int *abort_flag) {
-  return __all_sync(0xffffffffu, mbar_wait_for(bar, parity, limit_cycles, abort_flag)) != 0;
-}
-
 // Same contract, but polls with the non-suspending test_wait: lowest wake-up latency,
 // for pipelines whose stage hand-offs sit on the critical path.
 __device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {

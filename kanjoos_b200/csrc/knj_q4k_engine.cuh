@@ -350,9 +350,10 @@ __device__ __forceinline__ int job_locate(const int *jbase, int job) {
 // exists and names its output row (pair) and its activation row; load_row(row, sb, lane, v) fetches values
 // 256 sb + 8 lane .. + 7 of that activation row. out0/out1/out2 as for the launches: DUAL -> G, U, silu(G) * U;
 // otherwise out0 = Y. Bit s of `parity` is the phase the warp's next wait on its barrier s expects (0 after
-// initialisation); `ok` turns false when a wait of this warp gave up (the rest of the phase is then skipped, the CTA
-// barriers are still met). Other warps may have landed all their boxes: what a CTA reports is *sm.fail, read behind a
-// CTA barrier, not one warp's `ok`.
+// initialisation); `ok` turns false in a lane whose wait gave up: it waits, asks and stores no more, but goes through the
+// rest of the phase with its warp (the products are warp-wide instructions; sums of a box that did not land go nowhere) and
+// meets all barriers. Other lanes and warps may have landed all their boxes: what a CTA reports is *sm.fail, read behind a
+// CTA barrier, not a thread's `ok`.
 // ksplit (1, 2 or 4, a divisor of the boxes per tile): that many adjacent warps share a tile, each taking a
 // contiguous part of its K range; their partial sums meet in sm.red (fixed order, two named barriers per tile).
 // For runs with few tiles per warp, where a warp walking the whole K alone would be the critical path.
@@ -387,7 +388,7 @@ __device__ __forceinline__ void run_phase(const PhaseShape &sh, const PhaseSmem 
     // consumer has just left once the ring is full. No divisions in the loops below: counters only.
     int p_left = n_items, p_stage = 0, p_bl = 0, p_row = row_base;
     auto issue_next = [&]() {
-      if (lane == 0) {
+      if (lane == 0 && ok) {
         uint8_t *dst = ring + (size_t)p_stage * stage_bytes;
         const int x = (part * nb + p_bl) * (pitch / 4);
         fence_proxy_async();
@@ -402,7 +403,7 @@ __device__ __forceinline__ void run_phase(const PhaseShape &sh, const PhaseSmem 
       }
       --p_left;
     };
-    if (ok && trace_mode != 2)
+    if (trace_mode != 2)
       for (int i = 0; i < S && p_left > 0; ++i) issue_next();
 
     __syncthreads();  // the previous job's tiles are done with the panels
@@ -432,42 +433,38 @@ __device__ __forceinline__ void run_phase(const PhaseShape &sh, const PhaseSmem 
       const uint8_t *pan = sm.panels + (size_t)sb_first * kPanelBytes;
       const float *inv = sm.inv + (PL == 1 ? 2 * t : t) * 16 + sb_first;
       for (int bl = 0; bl < nb; ++bl) {
-        if (ok) {
-          bool landed = true;
-          if (trace_mode != 2) {
-            landed = mbar_wait_warp(&bars[stage], (parity >> stage) & 1u, wait_cycles, sm.fail);
-            parity ^= 1u << stage;
-          }
-          if (trace_mode != 1) {  // not asked about `landed` yet (the vote's latency): sums of a box that did not land go nowhere
-            const uint8_t *src = ring + (size_t)stage * stage_bytes;
-            for (int k = 0; k < sbs; ++k, src += KNJ_Q4K_BYTES, pan += kPanelBytes, ++inv) {
-              auto nothing = [] {};
-              if constexpr (PL == 1) {
-                float pg[2], ph[2];
-                tile_part<1, 1>(src, pitch, wrow, pan, tok_stride, lane, pg, ph, nothing);
-                rg[0] = fmaf(pg[0], inv[0], rg[0]);
-                rh[0] = fmaf(ph[0], inv[0], rh[0]);
-                rg[1] = fmaf(pg[1], inv[16], rg[1]);
-                rh[1] = fmaf(ph[1], inv[16], rh[1]);
-              } else if (two) {
-                float pg[2], ph[2];
-                tile_part<2>(src, pitch, wrow, pan, tok_stride, lane, pg, ph, nothing);
-                rg[0] = fmaf(pg[0], inv[0], rg[0]);
-                rh[0] = fmaf(ph[0], inv[0], rh[0]);
-                rg[1] = fmaf(pg[1], inv[64], rg[1]);
-                rh[1] = fmaf(ph[1], inv[64], rh[1]);
-              } else {
-                float pg[1], ph[1];
-                tile_part<1>(src, pitch, wrow, pan, tok_stride, lane, pg, ph, nothing);
-                rg[0] = fmaf(pg[0], inv[0], rg[0]);
-                rh[0] = fmaf(ph[0], inv[0], rh[0]);
-              }
+        if (trace_mode != 2) {
+          if (ok && !mbar_wait_for(&bars[stage], (parity >> stage) & 1u, wait_cycles, sm.fail)) ok = false;
+          parity ^= 1u << stage;
+        }
+        if (trace_mode != 1) {
+          const uint8_t *src = ring + (size_t)stage * stage_bytes;
+          for (int k = 0; k < sbs; ++k, src += KNJ_Q4K_BYTES, pan += kPanelBytes, ++inv) {
+            auto nothing = [] {};
+            if constexpr (PL == 1) {
+              float pg[2], ph[2];
+              tile_part<1, 1>(src, pitch, wrow, pan, tok_stride, lane, pg, ph, nothing);
+              rg[0] = fmaf(pg[0], inv[0], rg[0]);
+              rh[0] = fmaf(ph[0], inv[0], rh[0]);
+              rg[1] = fmaf(pg[1], inv[16], rg[1]);
+              rh[1] = fmaf(ph[1], inv[16], rh[1]);
+            } else if (two) {
+              float pg[2], ph[2];
+              tile_part<2>(src, pitch, wrow, pan, tok_stride, lane, pg, ph, nothing);
+              rg[0] = fmaf(pg[0], inv[0], rg[0]);
+              rh[0] = fmaf(ph[0], inv[0], rh[0]);
+              rg[1] = fmaf(pg[1], inv[64], rg[1]);
+              rh[1] = fmaf(ph[1], inv[64], rh[1]);
+            } else {
+              float pg[1], ph[1];
+              tile_part<1>(src, pitch, wrow, pan, tok_stride, lane, pg, ph, nothing);
+              rg[0] = fmaf(pg[0], inv[0], rg[0]);
+              rh[0] = fmaf(ph[0], inv[0], rh[0]);
             }
           }
-          __syncwarp();  // every lane is done with the box
-          ok = landed;
-          if (ok && trace_mode != 2 && p_left > 0) issue_next();
         }
+        __syncwarp();  // every lane is done with the box
+        if (trace_mode != 2 && p_left > 0) issue_next();
         if (++stage == S) stage = 0;
       }
       bool mine = true;

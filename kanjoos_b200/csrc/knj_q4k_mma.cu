@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_proj_kernel(const __grid_cons
       },
       [&](int row, int sb, int ln, float (&v)[8]) { q4e::load8_f32(p.X, p.x_dtype, (int64_t)row * p.ldx + 256 * sb + 8 * ln, v); },
       tmode);
-  if (!ok && lane == 0 && p.status) atomicExch(p.status, 1);
+  if (!ok && p.status) atomicExch(p.status, 1);
   if (IDENT) {
     // A dense product has no status word: where a wait gave up, all outputs of this CTA's units become NaN, so that a
     // caller cannot take what the buffer held before for a result.

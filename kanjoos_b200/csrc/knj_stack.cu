@@ -398,14 +398,14 @@ __device__ __noinline__ void stage_down_q6k(const StackParams &p, const LayerDes
     const int r0 = max(u0, job * tiles), r1 = min(u1, (job + 1) * tiles);
     const uint8_t *src = L.w_down6 + ((size_t)e * H - (size_t)job * tiles * 16) * (tb / 16);
     auto issue = [&](int tile) {
-      if (lane == 0) {
+      if (lane == 0 && ok) {
         fence_proxy_async();  // the buffer was read through the generic proxy
         mbar_expect_tx(bar, tb);
         bulk_g2s(buf, src + (size_t)tile * tb, tb, bar);
       }
     };
     int tile = warp < nw ? r0 + warp : r1;
-    if (ok && tile < r1) issue(tile);
+    if (tile < r1) issue(tile);
     __syncthreads();  // the previous job's tiles are done with the panel
     // ---- the job's tokens: the (4 (job - first job of the expert))-th and following of the expert's set
     for (int item = warp; item < q4e::kJobTok * nsb; item += q4e::kWarps) {
@@ -425,20 +425,17 @@ __device__ __noinline__ void stage_down_q6k(const StackParams &p, const LayerDes
     }
     __syncthreads();
     for (; tile < r1; tile += nw) {
-      if (ok) {
-        const bool landed = mbar_wait_warp(bar, parity & 1u, p.wait_cycles, fail);
-        parity ^= 1u;
-        float y0, y1;
-        q6b::tile_mma(buf, panel, inv + t * 16, nsb, lane, y0, y1);  // not asked about `landed` yet: as in run_phase
-        __syncwarp();  // every lane is done with the buffer
-        ok = landed;
-        if (ok && tile + nw < r1) issue(tile + nw);
-        const int pair = s_pair[t];
-        if (ok && pair >= 0) {
-          float *y = p.Y + (size_t)pair * H + (tile - job * tiles) * 16 + g;
-          y[0] = y0;
-          y[8] = y1;
-        }
+      if (ok && !mbar_wait_for(bar, parity & 1u, p.wait_cycles, fail)) ok = false;
+      parity ^= 1u;
+      float y0, y1;
+      q6b::tile_mma(buf, panel, inv + t * 16, nsb, lane, y0, y1);  // whatever each lane's wait came to: as in run_phase
+      __syncwarp();  // every lane is done with the buffer
+      if (tile + nw < r1) issue(tile + nw);
+      const int pair = s_pair[t];
+      if (ok && pair >= 0) {
+        float *y = p.Y + (size_t)pair * H + (tile - job * tiles) * 16 + g;
+        y[0] = y0;
+        y[8] = y1;
       }
     }
   }
